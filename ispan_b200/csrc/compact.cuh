@@ -177,8 +177,7 @@ __global__ void __launch_bounds__(kBlock) k_cmp_offsets(Run<OffT> r, Ext<OffT> x
     }
 }
 
-// adjacency in compact ids (input order kept), and the large-WCC list in
-// compact ids
+// adjacency in compact ids (input order kept)
 template <typename OffT>
 __global__ void __launch_bounds__(kBlock) k_cmp_fill(Run<OffT> r, Ext<OffT> x, CmpBufs b) {
     pdl_wait();  // predecessor done, its writes visible
@@ -197,7 +196,6 @@ __global__ void __launch_bounds__(kBlock) k_cmp_fill(Run<OffT> r, Ext<OffT> x, C
             const int32_t w = ld_adj(r.bw_adj, e);
             if (w != v && bitc(r.A, w)) b.badj[p++] = __ldcg(b.newid + w);
         }
-        x.large[0][i] = (int32_t)i;
     }
 }
 

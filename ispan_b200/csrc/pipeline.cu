@@ -30,6 +30,7 @@
 #include "pack.cuh"
 #include "transpose.cuh"
 #include "compact.cuh"
+#include "resolve.cuh"
 #include "tiny.cuh"
 #include "lane.h"
 #include "stages.cuh"
@@ -173,7 +174,7 @@ struct ispan_ctx {
 
     // launch geometry
     int g_stream = 0;           // grid for plain grid-stride kernels
-    int g_coop[5] = {0, 0, 0, 0, 0};  // bfs<0>, bfs<1>, trim1, color, color on the compact graph
+    int g_coop[5] = {0, 0, 0, 0, 0};  // bfs<0>, bfs<1>, trim1, color, split and resolve
     int g_pair = 0;             // each search's grid when the two run at the same time
 
     // the backward search's stream when the searches run at the same time
@@ -433,7 +434,6 @@ static void compact_run(const Run<OffT> &r, const Ext<OffT> &x, const CmpBufs &b
     xc.cq[0] = x.cq[0];
     xc.cq[1] = x.cq[1];
     xc.cand = x.cand;
-    xc.old = b.old;
 }
 
 // A plain launch, with programmatic stream serialization when pdl is set.
@@ -597,7 +597,7 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
         // once the degrees they hold are scanned), 2 (maxV + 32) entries each
         b.fadj = c->wl[0];
         b.badj = c->members;
-        b.bsum = reinterpret_cast<long long *>(c->aux);
+        b.bsum = reinterpret_cast<long long *>(c->large[1]);
         b.cap_e = 2 * (c->maxV + 32);
         b.V = r.V;
         const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(kScanBlocks, r.V / 4));
@@ -608,7 +608,39 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
         Run<int32_t> rc;
         Ext<int32_t> xc;
         compact_run(r, x, b, rc, xc);
-        if ((e = launch_coop(k_color<int32_t>, c->g_coop[4], s, rc, xc))) return e;
+        ResBufs m;
+        m.beg[0] = b.bbeg;
+        m.beg[1] = b.fbeg;
+        m.adj[0] = b.badj;
+        m.adj[1] = b.fadj;
+        m.end[0] = reinterpret_cast<int32_t *>(c->qe[0]);
+        m.end[1] = m.end[0] + r.V;
+        m.old = b.old;
+        m.parent = c->parent;  // WCC roots and, at them, sizes: as the WCC stage left them
+        m.wsize = c->aux;
+        m.val[0] = reinterpret_cast<uint32_t *>(c->aux2);
+        m.val[1] = reinterpret_cast<uint32_t *>(c->parent);
+        m.cls = reinterpret_cast<uint32_t *>(c->cnt_in);
+        m.mn = c->aux;
+        m.size = c->cnt_out;  // the compact ids of the build are no longer needed
+        m.list[0] = c->large[0];
+        m.list[1] = c->large[1];
+        m.q[0] = reinterpret_cast<uint32_t *>(c->qv[0]);
+        m.q[1] = reinterpret_cast<uint32_t *>(c->qv[1]);
+        m.cap_q = r.V;
+        m.order = reinterpret_cast<int32_t *>(m.q[1]);
+        m.pos = reinterpret_cast<int32_t *>(m.val[0]);
+        for (int it = 0; it < kResIts; ++it) {
+            if ((e = launch_coop(k_split, c->g_coop[4], s, rc, xc, m, it))) return e;
+            cudaLaunchConfig_t cfg;
+            memset(&cfg, 0, sizeof cfg);
+            cfg.gridDim = dim3((unsigned)c->nsm);
+            cfg.blockDim = dim3(kTileThreads);
+            cfg.dynamicSmemBytes = sizeof(TileSmem);
+            cfg.stream = s;
+            if ((e = cudaLaunchKernelEx(&cfg, k_tiles, rc, xc, m, it))) return e;
+        }
+        if ((e = launch_coop(k_resolve, c->g_coop[4], s, rc, xc, m))) return e;
         prev_plain = false;
     }
     if ((e = launch_coop(k_color<OffT>, c->g_coop[3], s, r, x))) return e;
@@ -639,7 +671,8 @@ static int coop_setup(ispan_ctx *c) {
     c->g_pair = std::max(1, std::min(c->g_coop[0], c->g_coop[1]) / 2);
     c->g_coop[2] = coop_grid(k_trim1<OffT>, nsm, kBlock);
     c->g_coop[3] = coop_grid(k_color<OffT>, nsm, kBlock);
-    c->g_coop[4] = coop_grid(k_color<int32_t>, nsm, kBlock);
+    c->g_coop[4] = std::min(coop_grid(k_split, nsm, kBlock), coop_grid(k_resolve, nsm, kBlock));
+    CK(cudaFuncSetAttribute(k_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
     for (int i = 0; i < 5; ++i)
         if (c->g_coop[i] < 1) return ISPAN_ERR_CUDA;
     c->g_coop_w = w;

@@ -24,8 +24,17 @@ enum Ctl64 {
     K_CMP_OK, K_CMP_EF, K_CMP_EB,  // compact colouring graph: built (1), its edge counts
     K_WCC_GIANT,                   // (root << 32) | 1 when one WCC holds half the root sample
     K_TINY,                        // 1: k_tiny_residual solved the residual; later stages return at once
-    kNumCtl = 32
+    K_RES_CHG,                     // k_resolve (resolve.cuh): values changed in a pass (3 slots),
+    K_RES_Q = K_RES_CHG + 3,       // vertices listed for the next level (3 slots),
+    K_RES_LEFT = K_RES_Q + 3,      // vertices left after a round (3 slots),
+    K_RES_STOP = K_RES_LEFT + 3,   // 1: no more splitting
+    K_RES_WORK,                    // the tiles' work (3 x kResWork, see ResWork)
+    kNumCtl = 64
 };
+
+// what k_split leaves for k_tiles: vertices in tiles of components, components
+// with a tile of their own, their vertices, next tile
+enum ResWork { W_SMALL = 0, W_MID, W_BACK, W_TILE, kResWork };
 
 constexpr int kLocalV = 1024;   // a WCC up to this many vertices ...
 constexpr int kLocalE = 4096;   // ... and internal edges is solved in shared memory
@@ -38,15 +47,7 @@ struct Ext {
     int32_t *large[2];            // [V] vertices of large WCCs (double buffered)
     int32_t *cq[2];               // [V] peel cascade queues
     int32_t *cand;                // [V] trim-2/3 candidates left by the first peel (count K_CAND)
-    const int32_t *old;           // colouring on the compact graph: original id of each compact id
-                                  // (NULL: the colouring runs on the input graph's ids)
 };
-
-// original vertex id of a colouring vertex id
-template <typename OffT>
-__device__ __forceinline__ int32_t orig_id(const Ext<OffT> &x, int32_t v) {
-    return x.old ? __ldg(x.old + v) : v;
-}
 
 // ---------------------------------------------------------------------------
 // Block-level compaction of bitmap words into a worklist with one atomic per
@@ -648,6 +649,19 @@ __global__ void __launch_bounds__(kBlock) k_wcc_init(Run<OffT> r, Ext<OffT> x, i
             r.D[w] = 0u;
 }
 
+// join the trees of a and b: the larger root goes under the smaller one
+__device__ __forceinline__ void uf_hook(int32_t *parent, int32_t a, int32_t b) {
+    for (int guard = 0; guard < (1 << 20); ++guard) {
+        a = uf_find(parent, a);
+        b = uf_find(parent, b);
+        if (a == b) break;
+        if (a > b) { int32_t t = a; a = b; b = t; }
+        int32_t old = atomicCAS(parent + b, b, a);  // hook root b under a
+        if (old == b) break;
+        b = old;
+    }
+}
+
 // hook the active neighbours adj[e0, e1) of v (four ids, then their active
 // bits, in flight together)
 __device__ __forceinline__ void hook_range(int32_t *parent, const uint32_t *A, const int32_t *adj, int32_t v,
@@ -662,16 +676,7 @@ __device__ __forceinline__ void hook_range(int32_t *parent, const uint32_t *A, c
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             if (!act[q]) continue;
-            int32_t a = v, b = ws[q];
-            for (int guard = 0; guard < (1 << 20); ++guard) {
-                a = uf_find(parent, a);
-                b = uf_find(parent, b);
-                if (a == b) break;
-                if (a > b) { int32_t t = a; a = b; b = t; }
-                int32_t old = atomicCAS(parent + b, b, a);  // hook root b under a
-                if (old == b) break;
-                b = old;
-            }
+            uf_hook(parent, v, ws[q]);
         }
     }
 }
@@ -1469,9 +1474,8 @@ __device__ __forceinline__ int color_async(const Run<OffT> &r, const Ext<OffT> &
     return -1;
 }
 
-// Runs on the input graph's ids (x.old NULL) unless the compact graph was
-// built, or on the compact graph (x.old set, r holding its CSR) if it was;
-// the pipeline launches both forms and one of them returns at once.
+// Runs on the input graph unless the compact graph was built (k_resolve has
+// taken its vertices then).
 template <typename OffT>
 #ifndef ISPAN_COLOR_MIN_CTAS
 #define ISPAN_COLOR_MIN_CTAS 2  // CTAs per SM the colouring kernel is compiled for (registers: 64 at 2)
@@ -1481,7 +1485,7 @@ __global__ void __launch_bounds__(kBlock, ISPAN_COLOR_MIN_CTAS) k_color(Run<OffT
     pdl_trigger();
     __shared__ int64_t sh[kWarps];
     __shared__ ColorSmem sm;
-    if ((__ldcg(x.ctl + K_CMP_OK) != 0) != (x.old != nullptr)) return;
+    if (__ldcg(x.ctl + K_CMP_OK) != 0) return;
     const int64_t gt = (int64_t)blockIdx.x * kBlock + threadIdx.x;
     const int64_t nt = (int64_t)gridDim.x * kBlock;
     // class (high half) and colour (low half) of each vertex in one word
@@ -1500,14 +1504,13 @@ __global__ void __launch_bounds__(kBlock, ISPAN_COLOR_MIN_CTAS) k_color(Run<OffT
         if (blockIdx.x == 0 && threadIdx.x == 0) x.ctl[K_MINPRIO0] = ~0ull;
         if (n == 0) return;
         // every word dead first: neighbours outside the large WCCs fail the class
-        // compare (the compact graph has no such neighbours; its ids are < n)
-        const int64_t nw = x.old ? n : r.V;
-        for (int64_t i = gt; i < nw; i += nt) cc[i] = kDeadWord;
+        // compare
+        for (int64_t i = gt; i < r.V; i += nt) cc[i] = kDeadWord;
         if (!grid_sync(r.gsync, r.err)) return;
         uint32_t pm = 0xffffffffu;
         for (int64_t i = gt; i < n; i += nt) {
             int32_t v = x.large[0][i];
-            cc[v] = ((unsigned long long)(uint32_t)r.parent[orig_id(x, v)] << 32) |
+            cc[v] = ((unsigned long long)(uint32_t)r.parent[v] << 32) |
                     ((unsigned long long)kNoColour << 1) | 1ull;
             pm = min(pm, prio_of((uint32_t)v));
         }
@@ -1574,7 +1577,7 @@ __global__ void __launch_bounds__(kBlock, ISPAN_COLOR_MIN_CTAS) k_color(Run<OffT
                 if (rt) {
                     set_bit(r.F, v);
                     rootof[v] = v;
-                    mn[v] = orig_id(x, v);
+                    mn[v] = v;
                     szc[v] = 0;
                 }
             }
@@ -1592,8 +1595,7 @@ __global__ void __launch_bounds__(kBlock, ISPAN_COLOR_MIN_CTAS) k_color(Run<OffT
             t[2] = npiv;
             t[3] = (long long)globaltimer();
         }
-        // a marked vertex's root is a vertex id (compact ids are smaller
-        // still); anything else is an internal error, recorded, and the
+        // a marked vertex's root is a vertex id; anything else is an internal error, recorded, and the
         // access skipped (the root tables hold V entries)
         const int64_t idb = r.V;
         for (int64_t i = gt; i < n; i += nt) {  // minimum member id and size per SCC
@@ -1604,7 +1606,7 @@ __global__ void __launch_bounds__(kBlock, ISPAN_COLOR_MIN_CTAS) k_color(Run<OffT
                     atomicCAS(r.err, 0, kErrOverflow);
                     continue;
                 }
-                atomicMin(mn + rv, orig_id(x, v));  // labels are original ids
+                atomicMin(mn + rv, v);
                 atomicAdd(szc + rv, 1);
             }
         }
@@ -1619,10 +1621,9 @@ __global__ void __launch_bounds__(kBlock, ISPAN_COLOR_MIN_CTAS) k_color(Run<OffT
                 if (bitv(r.F, v)) {
                     int32_t rv = __ldcg(rootof + v);
                     if ((uint64_t)(int64_t)rv >= (uint64_t)idb) rv = v;  // recorded above as an error
-                    const int32_t ov = orig_id(x, v);
-                    r.label[ov] = __ldcg(mn + rv);
-                    r.cls[ov] = CLS_MICE;
-                    clear_bit(r.A, ov);
+                    r.label[v] = __ldcg(mn + rv);
+                    r.cls[v] = CLS_MICE;
+                    clear_bit(r.A, v);
                     cc[v] = kDeadWord;
                     ++nl;
                     if (rv == v) {  // one histogram entry per SCC, at its root

@@ -1,0 +1,82 @@
+"""The splitting, tile and labelling kernels of the large WCCs (resolve.cuh) on
+graphs whose residual is built to reach their edges: components one vertex
+below, at and above the tile sizes, lists longer than a lane reads alone, a
+component too dense for a tile, duplicate edges and self-loops; exact labels
+against the oracle's Tarjan."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _csr(V, src, dst):
+    from ispan_b200.graphs import CSR
+    o = np.lexsort((dst, src))
+    s, d = src[o], dst[o]
+    fb = np.concatenate([[0], np.cumsum(np.bincount(s, minlength=V))]).astype(np.int64)
+    o = np.lexsort((src, dst))
+    bb = np.concatenate([[0], np.cumsum(np.bincount(dst, minlength=V))]).astype(np.int64)
+    return CSR(V, len(src), fb, d.astype(np.int32), bb, src[o].astype(np.int32))
+
+
+def _blocks(sizes, dag, seed, scramble, chords=0.5, dense=0):
+    """SCCs of the given sizes (ring and chords) in a line, joined by random
+    edges from earlier to later ones into one WCC, beside a strongly connected
+    hub graph (the pivot's SCC) and isolated vertices (four times the rest)."""
+    rng = np.random.default_rng(seed)
+    sizes = np.array(sizes)
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    n = int(off[-1])
+    of = np.repeat(np.arange(len(sizes)), sizes)
+    nxt = np.arange(1, n + 1)
+    nxt[off[1:] - 1] = off[:-1]
+    S, D = [np.arange(n)], [nxt]
+    c = rng.integers(0, n, int(n * chords))
+    S.append(c)
+    D.append(off[of[c]] + rng.integers(0, sizes[of[c]]))
+    x, y = rng.integers(0, n, dag), rng.integers(0, n, dag)
+    swap = of[x] > of[y]
+    S += [np.where(swap, y, x), np.arange(0, n, 97)]  # (the last: self-loops)
+    D += [np.where(swap, x, y), np.arange(0, n, 97)]
+    S.append(off[:-2])  # one WCC
+    D.append(off[1:-1])
+    if dense:  # the first block is dense, and a hub with long lists both ways
+        S += [rng.integers(0, sizes[0], dense), np.zeros(300, int), rng.integers(0, sizes[0], 300)]
+        D += [rng.integers(0, sizes[0], dense), rng.integers(0, n, 300), np.zeros(300, int)]
+    S.append(S[2][:500])  # duplicates
+    D.append(D[2][:500])
+    h = 1200  # the hub graph: one vertex to and from all others
+    S += [np.full(h, n), n + 1 + np.arange(h)]
+    D += [n + 1 + np.arange(h), np.full(h, n)]
+    V = 5 * (n + h + 1)
+    S, D = np.concatenate(S), np.concatenate(D)
+    if scramble:
+        p = rng.permutation(V)
+        S, D = p[S], p[D]
+    return _csr(V, S, D)
+
+
+CASES = {
+    "tile edges": dict(sizes=[2, 3, 1, 4095, 4096, 4097, 8191, 8192, 8193, 10000, 33] + [40] * 500, dag=60000),
+    "small": dict(sizes=[10] * 8000 + [700, 900], dag=160000),
+    "dense and hub": dict(sizes=[600] + [25] * 3000, dag=120000, dense=30000),
+    "rings": dict(sizes=[1000] * 90 + [7] * 100, dag=150000, chords=0.0),
+    "long ring": dict(sizes=[70000, 5, 5], dag=30, chords=0.0),
+    "nothing joins": dict(sizes=[3000] * 30, dag=0),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+@pytest.mark.parametrize("scramble", [False, True])
+def test_exact_labels(name, scramble):
+    import oracle
+    from ispan_b200 import Context
+    csr = _blocks(seed=len(name), scramble=scramble, **CASES[name])
+    exact = oracle.tarjan(csr)
+    with Context(csr.V, csr.E) as ctx:
+        for _ in range(2):
+            labels, st = ctx.run_csr(csr, histogram=True)
+            assert np.array_equal(labels, exact)
+            assert st["histogram"] == oracle.histogram(exact)
+            assert st["scc_count"] == len(np.unique(exact))
+            assert st["n_mice_vertices"] >= 65536  # the large-WCC path ran
