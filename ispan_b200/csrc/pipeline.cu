@@ -179,6 +179,8 @@ struct ispan_ctx {
 
     // the backward search's stream when the searches run at the same time
     cudaStream_t stream2 = nullptr;
+    // captures of the conditional parts of the graph, the inner one second
+    cudaStream_t stream_if[2] = {nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int g_coop_w = 0;           // offset width the coop grids were computed for
 
@@ -475,6 +477,39 @@ static bool pair_searches(const ispan_ctx *c, const Run<OffT> &r) {
     return t > 0 || r.V <= kPairMaxV;
 }
 
+// A part of the captured graph that runs only if its gate is open: if_gate
+// makes the gate (open unless a kernel closes it) in the graph that s is
+// captured into, if_begin adds the conditional node after what s captured so
+// far and starts capturing its body on sb, if_end goes on with s after it.
+static cudaError_t if_gate(cudaStream_t s, cudaGraphConditionalHandle *h) {
+    cudaStreamCaptureStatus st;
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamGetCaptureInfo_v3(s, &st, nullptr, &g, nullptr, nullptr, nullptr);
+    return e ? e : cudaGraphConditionalHandleCreate(h, g, 1, cudaGraphCondAssignDefault);
+}
+static cudaError_t if_begin(cudaStream_t s, cudaStream_t sb, cudaGraphConditionalHandle h, cudaGraphNode_t *node) {
+    cudaStreamCaptureStatus st;
+    cudaGraph_t g = nullptr;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t n = 0;
+    cudaError_t e = cudaStreamGetCaptureInfo_v3(s, &st, nullptr, &g, &deps, &edges, &n);
+    if (e) return e;
+    cudaGraphNodeParams p = {};
+    p.type = cudaGraphNodeTypeConditional;
+    p.conditional.handle = h;
+    p.conditional.type = cudaGraphCondTypeIf;
+    p.conditional.size = 1;
+    if ((e = cudaGraphAddNode_v2(node, g, deps, edges, n, &p))) return e;
+    return cudaStreamBeginCaptureToGraph(sb, p.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal);
+}
+static cudaError_t if_end(cudaStream_t s, cudaStream_t sb, cudaGraphNode_t node) {
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(sb, &g);
+    return e ? e : cudaStreamUpdateCaptureDependencies_v2(s, &node, nullptr, 1, cudaStreamSetCaptureDependencies);
+}
+
 // Enqueue the whole pipeline on c->stream (plain launches; may be captured).
 template <typename OffT>
 static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, bool capturing) {
@@ -482,6 +517,12 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     const int G = c->g_stream;
     unsigned long long *ctl = c->ctlblk;
     cudaError_t e;
+    // what follows the first peel, and in it the large WCCs, as conditional
+    // parts of a captured graph (stage times need their events between all
+    // stages, which a conditional part cannot hold)
+    const bool gates = capturing && !times && !(r.flags & ISPAN_F_EXACT_STATS);
+    cudaGraphNode_t if_left = nullptr, if_large = nullptr;
+    if (gates && (e = if_gate(s, &x.gate_left))) return e;
     const bool pair = pair_searches(c, r);
     if (pair) r.flags |= kRunPair;
     // a plain kernel that directly follows another plain kernel on s is
@@ -561,6 +602,11 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     prev_plain = false;
     if (r.flags & ISPAN_F_EXACT_STATS) PK((k_list_degrees<OffT>), G, kBlock, r, r.wl[1], x.ctl + K_WL1, C_Q2_N, C_Q2_XDEG);
     EV(5);
+    if (gates) {
+        if ((e = if_begin(s, c->stream_if[0], x.gate_left, &if_left))) return e;
+        s = c->stream_if[0];
+        if ((e = if_gate(s, &x.gate_large))) return e;
+    }
     PK((k_trim2<OffT>), G, kBlock, r, x, x.cand, x.ctl + K_CAND);
     EV(6);
     PK((k_trim3<OffT>), G, kBlock, r, x, x.cand, x.ctl + K_CAND);
@@ -583,6 +629,11 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     EV(9);
     PK((k_local_scc<OffT>), c->nsm * 6, kLocalThreads, r, x);
     EV(10);
+    if (gates) {
+        prev_plain = false;
+        if ((e = if_begin(s, c->stream_if[1], x.gate_large, &if_large))) return e;
+        s = c->stream_if[1];
+    }
     if (c->tuning.color_compact >= 0 && r.V >= 4 * kCmpMin) {  // (smaller graphs never qualify)
         // the large WCCs' subgraph in dense ids (compact.cuh), then the
         // colouring on it; the input-graph form returns at once if it was built
@@ -645,6 +696,11 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     }
     if ((e = launch_coop(k_color<OffT>, c->g_coop[3], s, r, x))) return e;
     prev_plain = false;
+    if (gates) {
+        if ((e = if_end(c->stream_if[0], s, if_large))) return e;
+        if ((e = if_end(c->stream, c->stream_if[0], if_left))) return e;
+        s = c->stream;
+    }
     EV(11);
     PK((k_finalize<OffT>), G, kBlock, r, x);
     EV(12);
@@ -711,8 +767,8 @@ static void l2_window(ispan_ctx *c, bool on) {
         v.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
         v.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
     }
-    if (cudaStreamSetAttribute(c->stream, cudaStreamAttributeAccessPolicyWindow, &v) != cudaSuccess)
-        cudaGetLastError();
+    for (cudaStream_t t : {c->stream, c->stream_if[0], c->stream_if[1]})
+        if (cudaStreamSetAttribute(t, cudaStreamAttributeAccessPolicyWindow, &v) != cudaSuccess) cudaGetLastError();
 }
 
 template <typename OffT>
@@ -782,6 +838,12 @@ static int run_t(ispan_ctx *c, int64_t V, int64_t E, int32_t nseg, const OffT *f
                 cudaError_t e2 = enqueue<OffT>(c, r, x, ev_on, true);
                 e = cudaStreamEndCapture(c->stream, &g);
                 if (e2 != cudaSuccess) e = e2;
+                for (cudaStream_t t : c->stream_if) {  // a part whose capture an error left open
+                    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+                    cudaGraph_t gi = nullptr;
+                    if (cudaStreamIsCapturing(t, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
+                        cudaStreamEndCapture(t, &gi);
+                }
             }
             if (e == cudaSuccess) e = cudaGraphInstantiate(&gx, g, 0);
             if (g) cudaGraphDestroy(g);
@@ -1480,6 +1542,8 @@ int ispan_ctx_create(int device, int64_t max_V, int64_t max_E, ispan_ctx **out) 
     if (!rc && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) rc = ISPAN_ERR_CUDA;
     c->own_stream = true;
     if (!rc && cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking) != cudaSuccess) rc = ISPAN_ERR_CUDA;
+    for (int i = 0; i < 2; ++i)
+        if (!rc && cudaStreamCreateWithFlags(&c->stream_if[i], cudaStreamNonBlocking) != cudaSuccess) rc = ISPAN_ERR_CUDA;
     if (!rc && (cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess))
         rc = ISPAN_ERR_CUDA;
@@ -1524,6 +1588,8 @@ int ispan_ctx_destroy(ispan_ctx *c) {
         cudaStreamSynchronize(c->stream2);
         cudaStreamDestroy(c->stream2);
     }
+    for (cudaStream_t t : c->stream_if)
+        if (t) cudaStreamDestroy(t);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     for (int k = 0; k < kUpChunks; ++k)
