@@ -106,6 +106,9 @@ constexpr int kHistCap = 1 << 16;   // exact histogram for SCC sizes below this
 constexpr int kTraceLevels = 256;   // levels recorded per search in the diagnostics trace
 constexpr int kBigCap = 1 << 16;    // list of larger SCC sizes (hist[kHistCap..])
 
+// classes recorded per vertex (for the reference-convention codes)
+enum Cls : uint8_t { CLS_NONE = 0, CLS_GIANT = 1, CLS_TRIM1 = 2, CLS_TRIM2 = 3, CLS_TRIM3 = 4, CLS_MICE = 5 };
+
 // error codes mirror ispan_b200.h
 constexpr int kErrTimeout = ISPAN_ERR_TIMEOUT;
 

@@ -440,12 +440,14 @@ static void compact_run(const Run<OffT> &r, const Ext<OffT> &x, const CmpBufs &b
 
 // A plain launch, with programmatic stream serialization when pdl is set.
 template <typename... P, typename... A>
-static cudaError_t launch_k(bool pdl, void (*k)(P...), int64_t grid, int block, cudaStream_t s, A... args) {
+static cudaError_t launch_k(bool pdl, void (*k)(P...), int64_t grid, int block, cudaStream_t s, size_t smem,
+                            A... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof cfg);
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
     cfg.stream = s;
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute at;
     memset(&at, 0, sizeof at);
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -535,7 +537,7 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
 #define LK(...) \
     do { __VA_ARGS__; e = cudaGetLastError(); if (e) return e; } while (0)
 #define PK(kern, grid, block, ...) \
-    do { e = launch_k(pdl_ok && prev_plain, kern, (grid), (block), s, __VA_ARGS__); if (e) return e; prev_plain = true; } while (0)
+    do { e = launch_k(pdl_ok && prev_plain, kern, (grid), (block), s, 0, __VA_ARGS__); if (e) return e; prev_plain = true; } while (0)
     EV(0);
     {   // every per-run counter, map and table that starts at zero, in one launch
         ResetDesc rd;
@@ -627,7 +629,9 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     PK((k_wcc_alloc<OffT>), G, kBlock, r, x);
     PK((k_wcc_scatter<OffT>), G, kBlock, r, x, 0);
     EV(9);
-    PK((k_local_scc<OffT>), c->nsm * 6, kLocalThreads, r, x);
+    if ((e = launch_k(pdl_ok && prev_plain, k_local_scc<OffT>, c->nsm * 2, LocalTile::kThreads, s, sizeof(LocalTile), r, x)))
+        return e;
+    prev_plain = true;
     EV(10);
     if (gates) {
         prev_plain = false;
@@ -728,6 +732,7 @@ static int coop_setup(ispan_ctx *c) {
     c->g_coop[2] = coop_grid(k_trim1<OffT>, nsm, kBlock);
     c->g_coop[3] = coop_grid(k_color<OffT>, nsm, kBlock);
     c->g_coop[4] = std::min(coop_grid(k_split, nsm, kBlock), coop_grid(k_resolve, nsm, kBlock));
+    CK(cudaFuncSetAttribute(k_local_scc<OffT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LocalTile)));
     CK(cudaFuncSetAttribute(k_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
     for (int i = 0; i < 5; ++i)
         if (c->g_coop[i] < 1) return ISPAN_ERR_CUDA;

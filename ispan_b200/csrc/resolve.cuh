@@ -37,6 +37,7 @@
 // here) 244 and 97 ms.
 #pragma once
 #include "compact.cuh"
+#include "tile.cuh"
 
 namespace ispan {
 
@@ -638,22 +639,9 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
 }
 
 // ---------------------------------------------------------------------------
-// The SCCs of small components in shared memory: a CTA takes a tile -- the
-// components that start in kTileT consecutive entries of m.order, or one
-// component of up to kTileV vertices -- as one graph of 16-bit local ids and
-// runs the labelling rounds of k_resolve on it: f and b both come from the
-// out-lists alone (f is pushed with atomicMin, b pulled by its owner), and a
-// label also jumps to the label of its holder, so a ring takes about
-// log(length) passes.
-struct TileSmem {
-    int32_t orig[kTileV];        // original ids
-    int32_t f[kTileV], b[kTileV];
-    uint16_t off[kTileV], len[kTileV];
-    uint16_t adj[kTileE];
-    uint32_t dead[kTileV / 32];
-    int32_t start, count, edges;
-    int64_t done, sccs;
-};
+// The components that start in kTileT consecutive entries of m.order, or one
+// component of up to kTileV vertices, as a tile (tile.cuh) of a CTA.
+using TileSmem = Tile<kTileV, kTileE, 1024>;
 constexpr int kTileThreads = 1024;
 constexpr int kTilePer = kTileV / kTileThreads;
 
@@ -668,7 +656,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Run<int32_t> r, Ext<i
     const int64_t n_small = (int64_t)__ldcg(work + W_SMALL), n_mid = (int64_t)__ldcg(work + W_MID);
     const int64_t tiles = (n_small + kTileT - 1) / kTileT;
     const int32_t *first = reinterpret_cast<const int32_t *>(m.val[1]);
-    if (tid == 0) { t.done = 0; t.sccs = 0; }
+    int64_t done = 0, sccs = 0;
     for (;;) {
         __syncthreads();  // the previous tile's readers are done
         if (tid == 0) {
@@ -748,126 +736,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Run<int32_t> r, Ext<i
                     if (w[q] >= 0) t.adj[o + k + q] = (uint16_t)(__ldcg(m.pos + w[q]) - start);
             }
         }
-        unsigned mine = 0;  // my vertices not solved yet
-#pragma unroll
-        for (int u = 0; u < kTilePer; ++u) mine |= (u * kTileThreads + tid < n ? 1u : 0u) << u;
-        int done = 0, sccs = 0;
-        for (int round = 0;; ++round) {
-            if (round > n) {  // every round finds the SCC of each class's lowest label
-                if (tid == 0) atomicCAS(r.err, 0, kErrOverflow);
-                break;
-            }
-            // (the barrier of the first test: lists and labels are in place)
-            // after k passes a label has come k edges far, so n passes are enough
-            int pass = 0;
-            for (int ch = 1; __syncthreads_or(ch); ++pass) {
-                if (pass > n + 2) {
-                    if (tid == 0) atomicCAS(r.err, 0, kErrOverflow);
-                    break;
-                }
-                ch = 0;
-#pragma unroll
-                for (int u = 0; u < kTilePer; ++u) {
-                    if (!((mine >> u) & 1u)) continue;
-                    const int i = u * kTileThreads + tid;
-                    volatile int32_t *f = t.f, *b = t.b;
-                    const int32_t f0 = f[i], b0 = b[i];
-                    const int32_t fv = min(f0, f[f0]);
-                    int32_t bv = min(b0, b[b0]);
-                    const int o = t.off[i], z = o + t.len[i];
-                    for (int k = o; k < z; ++k) {
-                        const int w = t.adj[k];
-                        if (f[w] > fv) { atomicMin(&t.f[w], fv); ch = 1; }
-                        bv = min(bv, b[w]);
-                    }
-                    if (fv < f0) { atomicMin(&t.f[i], fv); ch = 1; }
-                    if (bv < b0) { b[i] = bv; ch = 1; }
-                }
-            }
-            // solved: f = b = p.  A solved p gathers its SCC's lowest
-            // original id in f[p] and its size in b[p] (its members keep p in
-            // their own f)
-            unsigned sol = 0;
-#pragma unroll
-            for (int u = 0; u < kTilePer; ++u) {
-                const int i = u * kTileThreads + tid;
-                if (((mine >> u) & 1u) && t.f[i] == t.b[i]) sol |= 1u << u;
-            }
-            unsigned roots = 0;
-#pragma unroll
-            for (int u = 0; u < kTilePer; ++u)
-                if (((sol >> u) & 1u) && t.f[u * kTileThreads + tid] == u * kTileThreads + tid) roots |= 1u << u;
-            __syncthreads();
-#pragma unroll
-            for (int u = 0; u < kTilePer; ++u) {
-                const int i = u * kTileThreads + tid;
-                if ((sol >> u) & 1u) atomicOr(&t.dead[i >> 5], 1u << (i & 31));
-                if ((roots >> u) & 1u) {
-                    t.f[i] = t.orig[i];
-                    t.b[i] = 1;
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int u = 0; u < kTilePer; ++u) {
-                const int i = u * kTileThreads + tid;
-                if (((sol & ~roots) >> u) & 1u) {
-                    const int p = t.f[i];
-                    atomicMin(&t.f[p], t.orig[i]);
-                    atomicAdd(&t.b[p], 1);
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int u = 0; u < kTilePer; ++u) {
-                const int i = u * kTileThreads + tid;
-                if (!((sol >> u) & 1u)) continue;
-                const bool root = (roots >> u) & 1u;
-                const int32_t lab = root ? t.f[i] : t.f[t.f[i]], ov = t.orig[i];
-                r.label[ov] = lab;
-                r.cls[ov] = CLS_MICE;
-                clear_bit(r.A, ov);
-                ++done;
-                if (root) {
-                    atomicAdd((unsigned long long *)(r.hist + t.b[i]), 1ull);  // at most kTileV < kHistCap
-                    ++sccs;
-                }
-            }
-            mine &= ~sol;
-            // the others keep the entries of their own class (f, b)
-#pragma unroll
-            for (int u = 0; u < kTilePer; ++u) {
-                if (!((mine >> u) & 1u)) continue;
-                const int i = u * kTileThreads + tid;
-                const int32_t fv = t.f[i], bv = t.b[i];
-                const int o = t.off[i], z = o + t.len[i];
-                int q = o;
-                for (int k = o; k < z; ++k) {
-                    const int w = t.adj[k];
-                    if (!((t.dead[w >> 5] >> (w & 31)) & 1u) && t.f[w] == fv && t.b[w] == bv) t.adj[q++] = (uint16_t)w;
-                }
-                t.len[i] = (uint16_t)(q - o);
-            }
-            if (!__syncthreads_or(mine != 0u)) break;
-#pragma unroll
-            for (int u = 0; u < kTilePer; ++u)
-                if ((mine >> u) & 1u) {
-                    const int i = u * kTileThreads + tid;
-                    t.f[i] = i;
-                    t.b[i] = i;
-                }
-        }
-        const int64_t wd = warp_sum64(done), ws = warp_sum64(sccs);
-        if (lane == 0 && wd) {
-            atomicAdd((unsigned long long *)&t.done, (unsigned long long)wd);
-            atomicAdd((unsigned long long *)&t.sccs, (unsigned long long)ws);
-        }
+        tile_solve(t, n, r, done, sccs);
     }
-    __syncthreads();
-    if (tid == 0 && t.done) {
-        atomicAdd(r.counters + C_MICE_V, (unsigned long long)t.done);
-        atomicAdd(r.counters + C_MICE_SCC, (unsigned long long)t.sccs);
-    }
+        tile_report(r, done, sccs);
 }
 
 // Labelling rounds of the vertices that no tile took, to the end.

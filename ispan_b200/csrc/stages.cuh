@@ -11,11 +11,9 @@
 // launches, and the peel (trim-1) decides from counters, not observations.
 #pragma once
 #include "common.cuh"
+#include "tile.cuh"
 
 namespace ispan {
-
-// classes recorded per vertex (for the reference-convention codes)
-enum Cls : uint8_t { CLS_NONE = 0, CLS_GIANT = 1, CLS_TRIM1 = 2, CLS_TRIM2 = 3, CLS_TRIM3 = 4, CLS_MICE = 5 };
 
 // control-block slots (Run::ctl64): worklist and queue counters
 enum Ctl64 {
@@ -38,8 +36,8 @@ enum Ctl64 {
 // with a tile of their own, their vertices, next tile
 enum ResWork { W_SMALL = 0, W_MID, W_BACK, W_TILE, kResWork };
 
-constexpr int kLocalV = 1024;   // a WCC up to this many vertices ...
-constexpr int kLocalE = 4096;   // ... and internal edges is solved in shared memory
+constexpr int kLocalV = 1024;   // a WCC up to this many vertices is solved in shared memory
+constexpr int kLocalLane = 64;  // entries of a list a lane reads alone there
 
 template <typename OffT>
 struct Ext {
@@ -619,6 +617,13 @@ __global__ void __launch_bounds__(kBlock) k_trim3(Run<OffT> r, Ext<OffT> x, cons
     if (threadIdx.x == 0 && t) atomicAdd(r.counters + C_TRIM3, (unsigned long long)t);
 }
 
+// members per tile: short enough that a small residual spreads over the SMs
+__device__ __forceinline__ int wcc_tile(int64_t n) {
+    int t = kLocalV;
+    while (t > 128 && n < 148ll * t) t >>= 1;
+    return t;
+}
+
 // ---------------------------------------------------------------------------
 // Weakly connected components of the residual: hook-and-pointer-jump
 // union-find (replaces coloring_wcc, src/color_propagation.h:468-593, and the
@@ -661,6 +666,9 @@ __global__ void __launch_bounds__(kBlock) k_wcc_init(Run<OffT> r, Ext<OffT> x, i
         r.aux2[v] = -1;    // member base of a small WCC
         r.cnt_out[v] = 0;  // fill cursor
     }
+    const int64_t tiles = n / wcc_tile(n) + 1;  // first WCC of each tile of the member list
+    for (int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x; i < tiles; i += (int64_t)gridDim.x * kBlock)
+        x.large[1][i] = 0x7fffffff;
     // a batch's per-graph giant roots are marked in D (free after the peels)
     if (r.nseg > 1)
         for (int64_t w = (int64_t)blockIdx.x * kBlock + threadIdx.x; w < r.W; w += (int64_t)gridDim.x * kBlock)
@@ -845,19 +853,27 @@ __global__ void __launch_bounds__(kBlock) k_wcc_alloc(Run<OffT> r, Ext<OffT> x) 
     pdl_trigger();
     if (__ldcg(x.ctl + K_TINY)) return;  // the residual was solved in one CTA
     const int64_t n = (int64_t)__ldcg(x.ctl + K_ROOTS);
+    const int per = wcc_tile((int64_t)__ldcg(x.ctl + K_WL0));
     for (int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x; i - threadIdx.x < n;
          i += (int64_t)gridDim.x * kBlock) {
-        bool sm = false;
-        int32_t v = 0;
-        if (i < n) {
-            v = x.roots[i];
-            int32_t c = r.aux[v];
-            if (c <= kLocalV) {
-                r.aux2[v] = (int32_t)atomicAdd(x.ctl + K_ALLOC, (unsigned long long)c);
-                sm = true;
-            }
+        const int32_t v = i < n ? x.roots[i] : 0, c = i < n ? r.aux[v] : 0;
+        const int32_t cs = c <= kLocalV ? c : 0;
+        int32_t incl = cs;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(kFull, incl, o);
+            if (lane_id() >= o) incl += y;
         }
-        wl_append(sm, v, x.small, x.ctl + K_SMALL);
+        unsigned long long at = 0;
+        if (lane_id() == 31 && incl) at = atomicAdd(x.ctl + K_ALLOC, (unsigned long long)incl);
+        at = __shfl_sync(kFull, at, 31);
+        const unsigned sm = __ballot_sync(kFull, cs > 0);
+        if (lane_id() == 0 && sm) atomicAdd(x.ctl + K_SMALL, (unsigned long long)__popc(sm));
+        if (cs) {
+            const int32_t b = (int32_t)at + incl - cs;
+            r.aux2[v] = b;
+            atomicMin(x.large[1] + b / per, b);
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(r.counters + C_WCC, (unsigned long long)n);
 }
@@ -879,7 +895,7 @@ __global__ void __launch_bounds__(kBlock) k_wcc_scatter(Run<OffT> r, Ext<OffT> x
             if (b >= 0) {
                 int32_t k = atomicAdd(r.cnt_out + root, 1);
                 if (VOK((long long)b + k, 15)) r.members[b + k] = v;
-                r.cnt_in[v] = k;  // local index inside the WCC
+                r.cnt_in[v] = b + k;  // its place in the member list
             } else {
                 big = true;
             }
@@ -889,222 +905,150 @@ __global__ void __launch_bounds__(kBlock) k_wcc_scatter(Run<OffT> r, Ext<OffT> x
 }
 
 // ---------------------------------------------------------------------------
-// Small WCCs: one CTA per WCC builds the induced subgraph in shared memory
-// and runs an iterative Tarjan on it (linear time; the reference's
-// mice_fw_bw, src/fw_bw.h:1585-1691, runs one forward-backward search per
-// pivot instead).  A WCC whose internal edges exceed kLocalE spills to the
-// large (colouring) path.
-constexpr int kLocalThreads = 256;
+// Small WCCs (the reference's mice_fw_bw, src/fw_bw.h:1585-1691, runs one
+// forward-backward search per pivot instead): a CTA takes the WCCs that start
+// in wcc_tile() consecutive places of the member list as a tile (tile.cuh),
+// or, where their edges overflow it, one by one; a WCC whose own edges
+// overflow it spills to the large path.  A serial Tarjan per WCC that was not
+// one SCC, by one thread, took 782 us for 8 WCCs of a 23-graph batch, and
+// 5,320 rings with chords 169 us a breadth-first level at a time; as tiles they
+// take about 350 and 80 us.
+using LocalTile = Tile<2 * kLocalV, 12288, 512>;
 
 template <typename OffT>
-__global__ void __launch_bounds__(kLocalThreads) k_local_scc(Run<OffT> r, Ext<OffT> x) {
+__global__ void __launch_bounds__(LocalTile::kThreads) k_local_scc(Run<OffT> r, Ext<OffT> x) {
     pdl_wait();  // predecessor done, its writes visible
     pdl_trigger();
     if (__ldcg(x.ctl + K_TINY)) return;  // the residual was solved in one CTA
-    __shared__ int32_t gid[kLocalV];
-    __shared__ int32_t loff[kLocalV + 1];
-    __shared__ uint16_t ladj[kLocalE];
-    __shared__ int16_t idx[kLocalV], low[kLocalV], stk[kLocalV], csv[kLocalV];
-    __shared__ int32_t cse[kLocalV];
-    __shared__ uint8_t onst[kLocalV];
-    __shared__ uint32_t fwm[kLocalV / 32], bwm[kLocalV / 32], frm[2][kLocalV / 32];
-    __shared__ int s_flag, s_min, s_both;
-    __shared__ long long s_wq;
-    const int64_t nsmall = (int64_t)__ldcg(x.ctl + K_SMALL);
-    for (int guard = 0; guard < (1 << 30); ++guard) {
-        // dynamic assignment: large and small WCCs interleave across CTAs
-        __syncthreads();  // everyone is done with the previous WCC (and s_wq)
-        if (threadIdx.x == 0) s_wq = (long long)atomicAdd(x.ctl + K_LOCAL_NEXT, 1ull);
-        __syncthreads();
-        const int64_t wq = s_wq;
-        if (wq >= nsmall) break;
-        const int32_t root = x.small[wq];
-        const int32_t nv = r.aux[root];
-        if (!ICHK(nv >= 1 && nv <= kLocalV, 17, nv)) continue;
-        const int32_t base = r.aux2[root];
-        // per-vertex internal out-degree, then a vertex-order scan by warp 0
-        for (int i = threadIdx.x; i < nv; i += kLocalThreads) {
-            int32_t u = r.members[base + i];
-            gid[i] = u;
-            int32_t dcount = 0;
-            int64_t e0 = ld_off(r.fw_beg, u), e1 = ld_off(r.fw_beg, u + 1);
-            for (int64_t e = e0; e < e1; ++e) {
-                int32_t w = ld_adj(r.fw_adj, e);
-                dcount += (w != u) && bitc(r.A, w);
+    extern __shared__ __align__(16) unsigned char tile_raw[];
+    using T = LocalTile;
+    T &t = *reinterpret_cast<T *>(tile_raw);
+    const int tid = threadIdx.x, lane = lane_id();
+    const int64_t total = (int64_t)__ldcg(x.ctl + K_ALLOC);
+    const int per = wcc_tile((int64_t)__ldcg(x.ctl + K_WL0));
+    const int64_t tiles = (total + per - 1) / per;
+    const int32_t *first = x.large[1];
+    int64_t done = 0, sccs = 0;
+    for (;;) {
+        __syncthreads();  // the previous tile's readers are done
+        if (tid == 0) {
+            const int64_t k = (int64_t)atomicAdd(x.ctl + K_LOCAL_NEXT, 1ull);
+            int64_t a = 0, z = -1;
+            if (k < tiles) {
+                a = first[k];
+                z = total;
+                for (int64_t j = k + 1; j < tiles; ++j)
+                    if (first[j] != 0x7fffffff) { z = first[j]; break; }
+                if (a > z) a = z;  // no WCC starts here
             }
-            loff[i + 1] = dcount;
+            t.start = (int32_t)a;
+            t.count = (int32_t)(z - a);  // -1: no more work
         }
         __syncthreads();
-        if (threadIdx.x < 32) {
-            int32_t carry = 0;
-            if (threadIdx.x == 0) loff[0] = 0;
-            for (int b0 = 0; b0 < nv; b0 += 32) {
-                int i = b0 + threadIdx.x;
-                int32_t inc = i < nv ? loff[i + 1] : 0;
+        if (t.count < 0) break;
+        const int32_t a = t.start, z = a + t.count;
+        bool one = false;  // WCC by WCC
+        for (int32_t lo = a, hi = z; lo < z;) {
+            const int n = hi - lo;
+            __syncthreads();
+            if (tid == 0) t.edges = 0;
+            for (int i = tid; i < T::kV / 32; i += T::kThreads) t.dead[i] = 0u;
+            __syncthreads();
+            int32_t v[T::kPer];
+            for (int u = 0; u < T::kPer && u * T::kThreads < n; ++u) {
+                const int i = u * T::kThreads + tid;
+                v[u] = i < n ? r.members[lo + i] : -1;
+                const int64_t e0 = v[u] >= 0 ? ld_off(r.fw_beg, v[u]) : 0, e1 = v[u] >= 0 ? ld_off(r.fw_beg, v[u] + 1) : 0;
+                // the active neighbours: a lane reads a short list, the warp a long one
+                int32_t d = 0;
+                for (int64_t e = e0; e < min(e1, e0 + kLocalLane); e += 4) {
+                    int32_t w[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) w[q] = e + q < min(e1, e0 + kLocalLane) ? ld_adj(r.fw_adj, e + q) : v[u];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) d += w[q] != v[u] && bitc(r.A, w[q]);
+                }
+                for (unsigned g = __ballot_sync(kFull, e1 - e0 > kLocalLane); g; g &= g - 1) {
+                    const int l = __ffs(g) - 1;
+                    const int64_t le = __shfl_sync(kFull, e1, l);
+                    const int32_t lv = __shfl_sync(kFull, v[u], l);
+                    int c = 0;
+                    for (int64_t e = __shfl_sync(kFull, e0, l) + kLocalLane + lane; e < le; e += 32) {
+                        const int32_t w = ld_adj(r.fw_adj, e);
+                        c += w != lv && bitc(r.A, w);
+                    }
+                    c = __reduce_add_sync(kFull, c);
+                    if (lane == l) d += c;
+                }
+                int32_t incl = min(d, T::kE + 1);
+#pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    int32_t y = __shfl_up_sync(kFull, inc, o);
-                    if (lane_id() >= o) inc += y;
+                    const int32_t y = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += y;
                 }
-                if (i < nv) loff[i + 1] = carry + inc;
-                carry += __shfl_sync(kFull, inc, 31);
-            }
-        }
-        __syncthreads();
-        const int32_t tot = loff[nv];
-        if (tot > kLocalE) {
-            // spill: hand the whole WCC to the colouring path
-            for (int i = threadIdx.x; i < nv; i += kLocalThreads) {
-                unsigned long long p = atomicAdd(x.ctl + K_LARGE, 1ull);
-                if (VOK((long long)p, 16)) x.large[0][p] = gid[i];
-            }
-            if (threadIdx.x == 0) atomicAdd(r.counters + C_SPILL, 1ull);
-            __syncthreads();
-            continue;
-        }
-        // fill local adjacency (local ids from the scatter pass)
-        for (int i = threadIdx.x; i < nv; i += kLocalThreads) {
-            {
-                int32_t u = gid[i];
-                int32_t p = loff[i];
-                int64_t e0 = ld_off(r.fw_beg, u), e1 = ld_off(r.fw_beg, u + 1);
-                for (int64_t e = e0; e < e1; ++e) {
-                    int32_t w = ld_adj(r.fw_adj, e);
-                    if (w != u && bitc(r.A, w)) {
-                        int32_t li = r.cnt_in[w];
-                        if (ICHK(p < kLocalE && li >= 0 && li < nv, 14, ((long long)p << 32) | (li & 0xffffffff)))
-                            ladj[p++] = (uint16_t)li;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        // One forward and one backward search from local vertex 0, all threads
-        // on bitmaps in shared memory.  If both reach every vertex, the WCC is
-        // a single SCC (the common case for planted cycles with chords) and
-        // no serial work is needed.
-        const int nw = (nv + 31) >> 5;
-        for (int i = threadIdx.x; i < kLocalV / 32; i += kLocalThreads) {
-            fwm[i] = 0; bwm[i] = 0; frm[0][i] = 0; frm[1][i] = 0;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) { fwm[0] = 1u; frm[0][0] = 1u; bwm[0] = 1u; s_min = 0x7fffffff; }
-        __syncthreads();
-        for (int lv = 0, fc = 0; lv < kLocalV; ++lv, fc ^= 1) {  // forward, frontier push
-            __syncthreads();  // all threads have read s_flag and frm of the last level
-            if (threadIdx.x == 0) s_flag = 0;
-            for (int i = threadIdx.x; i < kLocalV / 32; i += kLocalThreads) frm[fc ^ 1][i] = 0;
-            __syncthreads();
-            for (int i = threadIdx.x; i < nv; i += kLocalThreads) {
-                if (!((frm[fc][i >> 5] >> (i & 31)) & 1u)) continue;
-                for (int e = loff[i]; e < loff[i + 1]; ++e) {
-                    int w = ladj[e];
-                    uint32_t bb = 1u << (w & 31);
-                    if (!(atomicOr(&fwm[w >> 5], bb) & bb)) {
-                        atomicOr(&frm[fc ^ 1][w >> 5], bb);
-                        s_flag = 1;
-                    }
+                int32_t at = 0;
+                if (lane == 31) at = atomicAdd(&t.edges, incl);
+                at = __shfl_sync(kFull, at, 31);
+                if (v[u] >= 0) {
+                    t.orig[i] = v[u];
+                    t.f[i] = i;
+                    t.b[i] = i;
+                    t.off[i] = (uint16_t)min(at + incl - d, 0xffff);
+                    t.len[i] = (uint16_t)min(d, 0xffff);
                 }
             }
             __syncthreads();
-            if (!s_flag) break;
-        }
-        for (int lv = 0; lv < kLocalV; ++lv) {  // backward, pull over out-edges
-            __syncthreads();
-            if (threadIdx.x == 0) s_flag = 0;
-            __syncthreads();
-            for (int i = threadIdx.x; i < nv; i += kLocalThreads) {
-                if ((bwm[i >> 5] >> (i & 31)) & 1u) continue;
-                for (int e = loff[i]; e < loff[i + 1]; ++e)
-                    if ((bwm[ladj[e] >> 5] >> (ladj[e] & 31)) & 1u) {
-                        atomicOr(&bwm[i >> 5], 1u << (i & 31));
-                        s_flag = 1;
-                        break;
+            if (t.edges > T::kE) {
+                const int32_t size = r.aux[r.parent[r.members[lo]]];  // of the first WCC
+                if (!one && size < n) {
+                    one = true;
+                    hi = lo + size;
+                    continue;
+                }
+                for (int i = tid; i - tid < n; i += T::kThreads)
+                    wl_append(i < n, i < n ? r.members[lo + i] : 0, x.large[0], x.ctl + K_LARGE);
+                if (tid == 0) {
+                    atomicAdd(r.counters + C_SPILL, 1ull);
+                    atomicAdd(r.counters + C_LOCAL_WCC, ~0ull);  // not one of those solved here
+                }
+            } else {
+                for (int u = 0; u < T::kPer && u * T::kThreads < n; ++u) {
+                    const int i = u * T::kThreads + tid;
+                    const int64_t e0 = v[u] >= 0 ? ld_off(r.fw_beg, v[u]) : 0, e1 = v[u] >= 0 ? ld_off(r.fw_beg, v[u] + 1) : 0;
+                    int32_t p = v[u] >= 0 ? t.off[i] : 0;
+                    for (int64_t e = e0; e < min(e1, e0 + kLocalLane); e += 4) {
+                        int32_t w[4], l[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) w[q] = e + q < min(e1, e0 + kLocalLane) ? ld_adj(r.fw_adj, e + q) : v[u];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) l[q] = w[q] != v[u] && bitc(r.A, w[q]) ? r.cnt_in[w[q]] - lo : -1;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (l[q] >= 0 && ICHK(l[q] < n && p < T::kE, 14, ((long long)p << 32) | l[q])) t.adj[p++] = (uint16_t)l[q];
                     }
-            }
-            __syncthreads();
-            if (!s_flag) break;
-        }
-        int both = 0;
-        for (int i = threadIdx.x; i < nw; i += kLocalThreads) {
-            uint32_t m = fwm[i] & bwm[i];
-            if (i == nw - 1 && (nv & 31)) m &= (1u << (nv & 31)) - 1u;
-            both += __popc(m);
-        }
-        for (int o = 16; o; o >>= 1) both += __shfl_xor_sync(kFull, both, o);
-        __syncthreads();
-        if (threadIdx.x == 0) s_both = 0;
-        __syncthreads();
-        if (lane_id() == 0) atomicAdd(&s_both, both);
-        for (int i = threadIdx.x; i < nv; i += kLocalThreads) atomicMin(&s_min, gid[i]);
-        __syncthreads();
-        if (s_both == nv) {  // single SCC
-            const int32_t mn = s_min;
-            for (int i = threadIdx.x; i < nv; i += kLocalThreads) {
-                r.label[gid[i]] = mn;
-                r.cls[gid[i]] = CLS_MICE;
-            }
-            if (threadIdx.x == 0) {
-                atomicAdd((unsigned long long *)(r.hist + nv), 1ull);  // nv <= kLocalV
-                atomicAdd(r.counters + C_MICE_SCC, 1ull);
-                atomicAdd(r.counters + C_MICE_V, (unsigned long long)nv);
-                atomicAdd(r.counters + C_LOCAL_WCC, 1ull);
-            }
-        } else if (threadIdx.x == 0) {
-            // iterative Tarjan over the local CSR
-            for (int i = 0; i < nv; ++i) { idx[i] = -1; onst[i] = 0; }
-            int counter = 0, sp = 0, nscc = 0;
-            for (int s0 = 0; s0 < nv; ++s0) {
-                if (idx[s0] != -1) continue;
-                int cp = 0;
-                csv[0] = (int16_t)s0; cse[0] = loff[s0]; cp = 1;
-                idx[s0] = low[s0] = (int16_t)counter++;
-                stk[sp++] = (int16_t)s0; onst[s0] = 1;
-                while (cp > 0) {
-                    int vv = csv[cp - 1];
-                    int e = cse[cp - 1];
-                    bool down = false;
-                    for (; e < loff[vv + 1]; ++e) {
-                        int w = ladj[e];
-                        if (idx[w] == -1) {
-                            cse[cp - 1] = e + 1;
-                            idx[w] = low[w] = (int16_t)counter++;
-                            stk[sp++] = (int16_t)w; onst[w] = 1;
-                            csv[cp] = (int16_t)w; cse[cp] = loff[w]; cp++;
-                            down = true;
-                            break;
-                        } else if (onst[w] && idx[w] < low[vv]) {
-                            low[vv] = idx[w];
+                    for (unsigned g = __ballot_sync(kFull, e1 - e0 > kLocalLane); g; g &= g - 1) {
+                        const int l = __ffs(g) - 1;
+                        const int64_t le = __shfl_sync(kFull, e1, l);
+                        const int32_t lv = __shfl_sync(kFull, v[u], l);
+                        int32_t lp = __shfl_sync(kFull, p, l);
+                        for (int64_t e = __shfl_sync(kFull, e0, l) + kLocalLane; e < le; e += 32) {
+                            const int32_t w = e + lane < le ? ld_adj(r.fw_adj, e + lane) : lv;
+                            const bool in = w != lv && bitc(r.A, w);
+                            const unsigned m = __ballot_sync(kFull, in);
+                            if (in) t.adj[lp + __popc(m & lanemask_lt())] = (uint16_t)(r.cnt_in[w] - lo);
+                            lp += __popc(m);
                         }
                     }
-                    if (down) continue;
-                    if (low[vv] == idx[vv]) {
-                        int32_t mn = 0x7fffffff, k = sp, sz = 0;
-                        do { --k; mn = min(mn, gid[stk[k]]); ++sz; } while (stk[k] != vv);
-                        while (sp > k) {
-                            int w = stk[--sp];
-                            onst[w] = 0;
-                            r.label[gid[w]] = mn;
-                            r.cls[gid[w]] = CLS_MICE;
-                        }
-                        atomicAdd((unsigned long long *)(r.hist + sz), 1ull);  // sz <= kLocalV
-                        ++nscc;
-                    }
-                    cp--;
-                    if (cp > 0) {
-                        int p = csv[cp - 1];
-                        if (low[vv] < low[p]) low[p] = low[vv];
-                    }
                 }
+                __syncthreads();
+                tile_solve(t, n, r, done, sccs);
             }
-            atomicAdd(r.counters + C_MICE_SCC, (unsigned long long)nscc);
-            atomicAdd(r.counters + C_MICE_V, (unsigned long long)nv);
-            atomicAdd(r.counters + C_LOCAL_WCC, 1ull);
+            lo = hi;
+            hi = one && lo < z ? lo + r.aux[r.parent[r.members[lo]]] : z;
         }
-        __syncthreads();
-        // the WCC is done: leave the active map
-        for (int i = threadIdx.x; i < nv; i += kLocalThreads) clear_bit(r.A, gid[i]);
-        __syncthreads();
     }
+    tile_report(r, done, sccs);
+    if (blockIdx.x == 0 && tid == 0) atomicAdd(r.counters + C_LOCAL_WCC, __ldcg(x.ctl + K_SMALL));
     if (threadIdx.x == 0) set_gate(x.gate_large, x.ctl + K_TICKET1, x.ctl + K_LARGE);
 }
 

@@ -19,7 +19,7 @@ def _csr(V, src, dst):
     return CSR(V, len(src), fb, d.astype(np.int32), bb, src[o].astype(np.int32))
 
 
-def _blocks(sizes, dag, seed, scramble, chords=0.5, dense=0):
+def _blocks(sizes, dag, seed, scramble, chords=0.5, dense=0, join=True):
     """SCCs of the given sizes (ring and chords) in a line, joined by random
     edges from earlier to later ones into one WCC, beside a strongly connected
     hub graph (the pivot's SCC) and isolated vertices (four times the rest)."""
@@ -38,11 +38,12 @@ def _blocks(sizes, dag, seed, scramble, chords=0.5, dense=0):
     swap = of[x] > of[y]
     S += [np.where(swap, y, x), np.arange(0, n, 97)]  # (the last: self-loops)
     D += [np.where(swap, x, y), np.arange(0, n, 97)]
-    S.append(off[:-2])  # one WCC
-    D.append(off[1:-1])
+    if join:  # one WCC
+        S.append(off[:-2])
+        D.append(off[1:-1])
     if dense:  # the first block is dense, and a hub with long lists both ways
         S += [rng.integers(0, sizes[0], dense), np.zeros(300, int), rng.integers(0, sizes[0], 300)]
-        D += [rng.integers(0, sizes[0], dense), rng.integers(0, n, 300), np.zeros(300, int)]
+        D += [rng.integers(0, sizes[0], dense), rng.integers(0, n if join else sizes[0], 300), np.zeros(300, int)]
     S.append(S[2][:500])  # duplicates
     D.append(D[2][:500])
     h = 1200  # the hub graph: one vertex to and from all others
@@ -56,6 +57,16 @@ def _blocks(sizes, dag, seed, scramble, chords=0.5, dense=0):
     return _csr(V, S, D)
 
 
+# WCCs below, at and above the limit of the shared-memory path, tiles whose
+# edges overflow (solved WCC by WCC) and a WCC whose own do (spilled)
+SMALL = {
+    "limits": dict(sizes=[1023, 1024, 1025, 2, 3, 1] + [4] * 700, dag=0),
+    "one tile": dict(sizes=[9, 5, 4], dag=0),
+    "dense": dict(sizes=[400] + [30] * 60, dag=0, dense=9000),
+    "overflow": dict(sizes=[500] + [600] * 4, dag=0, dense=14000),
+    "chords": dict(sizes=[100] * 30, dag=0, chords=9.0),
+}
+
 CASES = {
     "tile edges": dict(sizes=[2, 3, 1, 4095, 4096, 4097, 8191, 8192, 8193, 10000, 33] + [40] * 500, dag=60000),
     "small": dict(sizes=[10] * 8000 + [700, 900], dag=160000),
@@ -64,6 +75,20 @@ CASES = {
     "long ring": dict(sizes=[70000, 5, 5], dag=30, chords=0.0),
     "nothing joins": dict(sizes=[3000] * 30, dag=0),
 }
+
+
+@pytest.mark.parametrize("name", list(SMALL))
+@pytest.mark.parametrize("graph", [False, True])
+def test_small_wccs(name, graph):
+    import oracle
+    from ispan_b200 import Context
+    csr = _blocks(seed=len(name), scramble=True, join=False, **SMALL[name])
+    exact = oracle.tarjan(csr)
+    with Context(csr.V, csr.E) as ctx:
+        labels, st = ctx.run_csr(csr, histogram=True, use_graph=graph)
+    assert np.array_equal(labels, exact)
+    assert st["histogram"] == oracle.histogram(exact)
+    assert st["local_wcc"] == st["n_wcc"] - (name == "limits") - (name == "overflow")
 
 
 @pytest.mark.parametrize("name", list(CASES))
