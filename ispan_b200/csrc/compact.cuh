@@ -32,12 +32,18 @@ constexpr int kScanBlocks = 1024;  // blocks of the offset scans (at most; one C
 constexpr int64_t kCmpMin = 1 << 16;  // fewer colouring vertices than this: no compact graph (the
                                       // input graph's colour words of so few vertices stay in L2)
 
+constexpr int64_t kCmpMinRest = 1 << 10;
+
 // Whether the compact graph is worth building: enough colouring vertices,
 // and spread thinly over the id range (at most a quarter of it).  Where they
 // are dense -- a batch, whose graphs are contiguous id ranges -- the input
 // graph's words and lists are already local, and measured on the batched
 // workload the build cost more than the rounds gained.
-__device__ __forceinline__ bool cmp_wanted(int64_t n, int64_t V) { return n >= kCmpMin && 4 * n <= V; }
+// What k_super left (`rest`) has mostly fallen apart into components for
+// tiles: worth it from far fewer (64 K of a batch: 6.7 ms of colouring).
+__device__ __forceinline__ bool cmp_wanted(int64_t n, int64_t V, const unsigned long long *ctl) {
+    return n >= (__ldcg(ctl + K_SUP_LEFT) ? kCmpMinRest : kCmpMin) && 4 * n <= V;
+}
 
 struct CmpBufs {
     int32_t *newid;   // [V]
@@ -58,7 +64,7 @@ __global__ void __launch_bounds__(kBlock) k_cmp_count(Run<OffT> r, Ext<OffT> x, 
     pdl_trigger();
     __shared__ int64_t sh[kWarps];
     const int64_t n = (int64_t)__ldcg(x.ctl + K_LARGE);
-    if (!cmp_wanted(n, b.V)) return;
+    if (!cmp_wanted(n, b.V, x.ctl)) return;
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t i0 = min(n, (int64_t)blockIdx.x * per), i1 = min(n, i0 + per);
     int64_t so = 0, si = 0;
@@ -95,7 +101,7 @@ __global__ void __launch_bounds__(kScanBlocks) k_cmp_tops(unsigned long long *ct
     pdl_trigger();
     __shared__ long long wt[2][kScanBlocks / 32];
     const int64_t n = (int64_t)__ldcg(ctl + K_LARGE);
-    if (!cmp_wanted(n, b.V)) {
+    if (!cmp_wanted(n, b.V, ctl)) {
         if (threadIdx.x == 0) ctl[K_CMP_OK] = 0ull;
         return;
     }

@@ -32,6 +32,7 @@
 #include "compact.cuh"
 #include "resolve.cuh"
 #include "tiny.cuh"
+#include "cycles.cuh"
 #include "lane.h"
 #include "stages.cuh"
 
@@ -174,7 +175,7 @@ struct ispan_ctx {
 
     // launch geometry
     int g_stream = 0;           // grid for plain grid-stride kernels
-    int g_coop[5] = {0, 0, 0, 0, 0};  // bfs<0>, bfs<1>, trim1, color, split and resolve
+    int g_coop[7] = {0, 0, 0, 0, 0, 0, 0};  // bfs<0>, bfs<1>, trim1, color, split and resolve, cycles, super
     int g_pair = 0;             // each search's grid when the two run at the same time
 
     // the backward search's stream when the searches run at the same time
@@ -617,7 +618,21 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     if ((e = launch_coop(k_trim1<OffT>, c->g_coop[2], s, r, x, 1, 0, 0))) return e;
     prev_plain = false;
     EV(8);
-    PK((k_wcc_init<OffT>), G, kBlock, r, x, 0);
+    // cycles along near ids (cycles.cuh), in arrays the searches and peels are
+    // done with
+    CycBufs cy;
+    cy.par = c->wl[1];
+    cy.rep = c->qv[0];
+    cy.order = c->qv[1];
+    cy.size = reinterpret_cast<int32_t *>(c->qe[0]);
+    cy.skip = cy.size + (c->maxV + 32);
+    cy.key = reinterpret_cast<unsigned long long *>(c->qe[1]);
+    cy.single = c->members;
+    cy.q[0] = c->members;
+    cy.q[1] = c->roots;
+    if ((e = launch_coop(k_cycles<OffT>, c->g_coop[5], s, r, x, cy))) return e;
+    prev_plain = false;
+    PK((k_wcc_init<OffT>), G, kBlock, r, x, 0, (const int32_t *)cy.rep);
     PK((k_wcc_hook<OffT>), G, kBlock, r, x, 0, 0);
     PK((k_wcc_compress<OffT>), G, kBlock, r, x, 0);
     if (r.nseg > 1)
@@ -629,7 +644,7 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     PK((k_wcc_alloc<OffT>), G, kBlock, r, x);
     PK((k_wcc_scatter<OffT>), G, kBlock, r, x, 0);
     EV(9);
-    if ((e = launch_k(pdl_ok && prev_plain, k_local_scc<OffT>, c->nsm * 2, LocalTile::kThreads, s, sizeof(LocalTile), r, x)))
+    if ((e = launch_k(pdl_ok && prev_plain, k_local_scc<OffT>, c->nsm, kTileThreads, s, sizeof(TileSmem), r, x)))
         return e;
     prev_plain = true;
     EV(10);
@@ -638,6 +653,8 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
         if ((e = if_begin(s, c->stream_if[1], x.gate_large, &if_large))) return e;
         s = c->stream_if[1];
     }
+    if ((e = launch_coop(k_super<OffT>, c->g_coop[6], s, r, x, cy))) return e;
+    prev_plain = false;
     if (c->tuning.color_compact >= 0 && r.V >= 4 * kCmpMin) {  // (smaller graphs never qualify)
         // the large WCCs' subgraph in dense ids (compact.cuh), then the
         // colouring on it; the input-graph form returns at once if it was built
@@ -732,9 +749,11 @@ static int coop_setup(ispan_ctx *c) {
     c->g_coop[2] = coop_grid(k_trim1<OffT>, nsm, kBlock);
     c->g_coop[3] = coop_grid(k_color<OffT>, nsm, kBlock);
     c->g_coop[4] = std::min(coop_grid(k_split, nsm, kBlock), coop_grid(k_resolve, nsm, kBlock));
-    CK(cudaFuncSetAttribute(k_local_scc<OffT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LocalTile)));
+    CK(cudaFuncSetAttribute(k_local_scc<OffT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
     CK(cudaFuncSetAttribute(k_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
-    for (int i = 0; i < 5; ++i)
+    c->g_coop[5] = coop_grid(k_cycles<OffT>, nsm, kBlock);
+    c->g_coop[6] = coop_grid(k_super<OffT>, nsm, kBlock);
+    for (int i = 0; i < 7; ++i)
         if (c->g_coop[i] < 1) return ISPAN_ERR_CUDA;
     c->g_coop_w = w;
     return ISPAN_OK;

@@ -18,7 +18,7 @@
 //     in shared memory.  Larger ones are split again, kResIts times in all.
 //   Labelling (in a tile, and k_resolve for what is left): every vertex
 //     carries the lowest label among its ancestors, f, and among its
-//     descendants, b, inside its class (labels are distinct).  Where f = b =
+//     descendants, b, inside its class (labels are the ids).  Where f = b =
 //     the label of p, p reaches the vertex and is reached from it: the vertex
 //     is in p's SCC, found without a separate backward search.  At least the
 //     SCC of each class's lowest label is.  The others go on, classed by
@@ -56,9 +56,6 @@ constexpr int64_t kResSparse = 16;     // a pass that changed at most 1 / 16 of 
 constexpr uint32_t kResHash = 0x07ffffffu;  // class word while splitting: 27 bits of hash, 5 bits of log2 |WCC|
 constexpr uint32_t kResDead = 0xffffffffu;  // class word of a vertex whose SCC is known
 
-constexpr int kTileT = 4096;   // consecutive entries of the order whose components make a tile: components up to this many vertices
-constexpr int kTileV = 8192;   // vertices of a tile, at most (a component may begin at the tile's last entry)
-constexpr int kTileE = 24576;  // list entries of a tile, at most
 
 struct ResBufs {
     // the lists of vertex v, [beg[v], end[v]) of adj: [0] in-, [1] out-lists,
@@ -83,23 +80,6 @@ __device__ __forceinline__ uint32_t mix32(uint32_t h) {
     h *= 0x846ca68bu;
     h ^= h >> 16;
     return h;
-}
-
-// the inverse of prio_of: xor-shifts by 16 and 15 undone on 31 bits, odd
-// multipliers by their inverses mod 2^31 (Newton's iteration)
-__host__ __device__ constexpr uint32_t odd_inverse(uint32_t a) {
-    uint32_t y = a;
-    for (int i = 0; i < 5; ++i) y *= 2u - a * y;
-    return y;
-}
-__device__ __forceinline__ uint32_t vertex_of(uint32_t p) {
-    constexpr uint32_t i1 = odd_inverse(0x7feb352du), i2 = odd_inverse(0x846ca68bu);
-    p ^= p >> 16;
-    p = (p * i2) & 0x7fffffffu;
-    p ^= (p >> 15) ^ (p >> 30);
-    p = (p * i1) & 0x7fffffffu;
-    p ^= p >> 16;
-    return p;
 }
 
 // The value of a vertex: a mask of pivots while splitting (OR, 16 or 64 bits
@@ -156,7 +136,7 @@ __device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int3
     for (int u = 0; u < kResU; ++u) {
         nw[u] = own[u];
         if constexpr (K == R_MIN)
-            if (v[u] >= 0) nw[u] = min(own[u], __ldcg(val + vertex_of(own[u])));
+            if (v[u] >= 0) nw[u] = min(own[u], __ldcg(val + own[u]));
     }
     bool more = true;
     for (int step = 0; step < kResLane && more; step += 4) {
@@ -513,7 +493,9 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
     // half of its 126 MB): wider ones split more per round
     const bool wide = n <= kResWideN || n > kResNarrowN;
     const int bits = wide ? 6 : 4;  // log2 of the pivots per class aimed at
-    const int rounds_now = it ? 2 : wide ? 3 : 4;
+    // (what k_super left of the large WCCs has mostly fallen apart: its
+    // components first)
+    const int rounds_now = it ? 2 : __ldcg(x.ctl + K_SUP_LEFT) ? 0 : wide ? 3 : 4;
     if (gt < 3) { chg[gt] = 0ull; qc[gt] = 0ull; }
     for (int64_t i = gt; i < nl; i += nt) {
         int32_t root, size;
@@ -641,8 +623,6 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
 // ---------------------------------------------------------------------------
 // The components that start in kTileT consecutive entries of m.order, or one
 // component of up to kTileV vertices, as a tile (tile.cuh) of a CTA.
-using TileSmem = Tile<kTileV, kTileE, 1024>;
-constexpr int kTileThreads = 1024;
 constexpr int kTilePer = kTileV / kTileThreads;
 
 __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Run<int32_t> r, Ext<int32_t> x, ResBufs m, int it) {
@@ -682,24 +662,17 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Run<int32_t> r, Ext<i
         const int n = t.count, start = t.start;
         if (n < 0) break;
         if (n == 0) continue;
+        for (int i = tid; i < n; i += kTileThreads) t.f[i] = m.old[m.order[start + i]];
+        for (int i = tid; i < kTileV / 32; i += kTileThreads) t.dead[i] = 0u;
+        tile_sort(t, n);
         int32_t e0[kTilePer];  // the list of each of my vertices
-        int32_t v[kTilePer];
-#pragma unroll
-        for (int u = 0; u < kTilePer; ++u) {
+        for (int u = 0; u < kTilePer && u * kTileThreads < n; ++u) {
             const int i = u * kTileThreads + tid;
-            v[u] = i < n ? m.order[start + i] : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < kTilePer; ++u) {
-            const int i = u * kTileThreads + tid;
-            if (u * kTileThreads >= n) break;
             int32_t d = 0;
-            if (v[u] >= 0) {
-                e0[u] = m.beg[1][v[u]];
-                d = m.end[1][v[u]] - e0[u];
-                t.orig[i] = m.old[v[u]];
-                t.f[i] = i;
-                t.b[i] = i;
+            if (i < n) {
+                const int32_t v = m.order[start + t.b[i]];
+                e0[u] = m.beg[1][v];
+                d = m.end[1][v] - e0[u];
             }
             int32_t incl = d;
 #pragma unroll
@@ -710,12 +683,11 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Run<int32_t> r, Ext<i
             int32_t at = 0;
             if (lane == 31) at = atomicAdd(&t.edges, min(incl, kTileE + 1));  // (the sum of 32 lists stays far below 2^31)
             at = __shfl_sync(kFull, at, 31);
-            if (v[u] >= 0) {
+            if (i < n) {
                 t.off[i] = (uint16_t)min(at + incl - d, 0xffff);
                 t.len[i] = (uint16_t)min(d, 0xffff);
             }
         }
-        for (int i = tid; i < kTileV / 32; i += kTileThreads) t.dead[i] = 0u;
         __syncthreads();
         if (t.edges > kTileE) {  // too dense for a tile: the labelling rounds take it
             for (int i = tid; i - tid < n; i += kTileThreads)
@@ -733,7 +705,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Run<int32_t> r, Ext<i
                 for (int q = 0; q < 4; ++q) w[q] = k + q < d ? __ldcg(m.adj[1] + e0[u] + k + q) : -1;
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (w[q] >= 0) t.adj[o + k + q] = (uint16_t)(__ldcg(m.pos + w[q]) - start);
+                    if (w[q] >= 0) t.adj[o + k + q] = (uint16_t)t.f[__ldcg(m.pos + w[q]) - start];
             }
         }
         tile_solve(t, n, r, done, sccs);
@@ -747,7 +719,6 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
     pdl_trigger();
     if (!__ldcg(x.ctl + K_CMP_OK)) return;
     __shared__ ResSmem sm;
-    const int64_t n = (int64_t)__ldcg(x.ctl + K_LARGE);
     const int64_t gt = (int64_t)blockIdx.x * kBlock + threadIdx.x;
     const int64_t nt = (int64_t)gridDim.x * kBlock;
     unsigned long long *chg = x.ctl + K_RES_CHG, *qc = x.ctl + K_RES_Q, *left = x.ctl + K_RES_LEFT;
@@ -763,9 +734,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
         if (gt == 0) left[(k + 1) % 3] = 0ull;
         for (int64_t i = gt; i < nl; i += nt) {
             const int32_t v = list[i];
-            const uint32_t p = prio_of((uint32_t)v);
-            m.val[0][v] = p;
-            m.val[1][v] = p;
+            m.val[0][v] = (uint32_t)v;
+            m.val[1][v] = (uint32_t)v;
             m.mn[v] = 0x7fffffff;
             m.size[v] = 0;
         }
@@ -775,13 +745,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
             const int32_t v = list[i];
             const uint32_t f = __ldcg(m.val[0] + v);
             if (f == __ldcg(m.val[1] + v)) {
-                const uint32_t p = vertex_of(f);
-                if ((int64_t)p >= n) {  // labels are those of compact ids
-                    atomicCAS(r.err, 0, kErrOverflow);
-                    continue;
-                }
-                atomicMin(m.mn + p, m.old[v]);
-                atomicAdd(m.size + p, 1);
+                atomicMin(m.mn + f, m.old[v]);
+                atomicAdd(m.size + f, 1);
             }
         }
         if (!grid_sync(r.gsync, r.err)) return;
@@ -796,14 +761,13 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
                 if (keep) {
                     m.cls[v] = mix32(f ^ mix32(b)) & 0x7fffffffu;
                 } else {
-                    const uint32_t p = min(vertex_of(f), (uint32_t)(n - 1));
                     const int32_t ov = m.old[v];
-                    r.label[ov] = __ldcg(m.mn + p);
+                    r.label[ov] = __ldcg(m.mn + f);
                     r.cls[ov] = CLS_MICE;
                     clear_bit(r.A, ov);
                     m.cls[v] = kResDead;
                     ++done;
-                    if ((int32_t)p == v) {  // one histogram entry per SCC
+                    if ((int32_t)f == v) {  // one histogram entry per SCC
                         const int32_t sz = __ldcg(m.size + v);
                         if (sz < kHistCap) {
                             atomicAdd((unsigned long long *)(r.hist + sz), 1ull);

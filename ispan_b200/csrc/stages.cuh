@@ -28,15 +28,25 @@ enum Ctl64 {
     K_RES_STOP = K_RES_LEFT + 3,   // 1: no more splitting
     K_RES_WORK,                    // the tiles' work (3 x kResWork, see ResWork)
     K_TICKET0 = K_RES_WORK + 12,   // CTAs done with the first peel,
-    K_TICKET1,                     // with k_local_scc (see gate)
-    kNumCtl = 64
+    K_TICKET1,                     // with k_local_scc (see set_gate)
+    K_MID, K_MID_BACK,             // WCCs with a tile of their own, their vertices
+    K_CYC_ON, K_CYC_N, K_CYC_MEM, K_CYC_LEFT,  // cycles.cuh: cycles were looked for (2: most edges lead down),
+                                   // vertices on those found, places taken, vertices on none,
+    K_SUP_Q, K_SUP_LEFT = K_SUP_Q + 3,  // vertices to peel (3 slots), vertices left
+    kNumCtl = 72
 };
 
 // what k_split leaves for k_tiles: vertices in tiles of components, components
 // with a tile of their own, their vertices, next tile
 enum ResWork { W_SMALL = 0, W_MID, W_BACK, W_TILE, kResWork };
 
-constexpr int kLocalV = 1024;   // a WCC up to this many vertices is solved in shared memory
+// tiles of the shared-memory solver (tile.cuh): one CTA per SM
+constexpr int kTileT = 4096;   // components up to this many vertices share tiles: those that start in as many places
+constexpr int kTileV = 8192;   // vertices of a tile, at most (a component may begin at the last place)
+constexpr int kTileE = 45056;  // list entries of a tile, at most
+constexpr int kTileThreads = 1024;
+using TileSmem = Tile<kTileV, kTileE, kTileThreads>;
+constexpr int kLocalV = kTileV;  // a WCC up to this many vertices is solved in shared memory
 constexpr int kLocalLane = 64;  // entries of a list a lane reads alone there
 
 template <typename OffT>
@@ -619,8 +629,8 @@ __global__ void __launch_bounds__(kBlock) k_trim3(Run<OffT> r, Ext<OffT> x, cons
 
 // members per tile: short enough that a small residual spreads over the SMs
 __device__ __forceinline__ int wcc_tile(int64_t n) {
-    int t = kLocalV;
-    while (t > 128 && n < 148ll * t) t >>= 1;
+    int t = kTileT;
+    while (t > 256 && n <= 148ll * (t / 2)) t >>= 1;
     return t;
 }
 
@@ -654,14 +664,15 @@ __device__ __forceinline__ int32_t uf_root(const int32_t *parent, int32_t x) {
 }
 
 template <typename OffT>
-__global__ void __launch_bounds__(kBlock) k_wcc_init(Run<OffT> r, Ext<OffT> x, int in) {
+__global__ void __launch_bounds__(kBlock) k_wcc_init(Run<OffT> r, Ext<OffT> x, int in, const int32_t *rep) {
     pdl_wait();  // predecessor done, its writes visible
     pdl_trigger();
     if (__ldcg(x.ctl + K_TINY)) return;  // the residual was solved in one CTA
+    const bool cyc = __ldcg(x.ctl + K_CYC_ON) != 0;
     const int64_t n = (int64_t)__ldcg(x.ctl + K_WL0 + in);
     for (int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x; i < n; i += (int64_t)gridDim.x * kBlock) {
         int32_t v = r.wl[in][i];
-        r.parent[v] = v;
+        r.parent[v] = cyc ? rep[v] : v;  // a cycle's vertices are joined already, under its minimum
         r.aux[v] = 0;      // member count (valid at roots)
         r.aux2[v] = -1;    // member base of a small WCC
         r.cnt_out[v] = 0;  // fill cursor
@@ -852,12 +863,13 @@ __global__ void __launch_bounds__(kBlock) k_wcc_alloc(Run<OffT> r, Ext<OffT> x) 
     pdl_wait();  // predecessor done, its writes visible
     pdl_trigger();
     if (__ldcg(x.ctl + K_TINY)) return;  // the residual was solved in one CTA
-    const int64_t n = (int64_t)__ldcg(x.ctl + K_ROOTS);
-    const int per = wcc_tile((int64_t)__ldcg(x.ctl + K_WL0));
+    const int64_t n = (int64_t)__ldcg(x.ctl + K_ROOTS), nv = (int64_t)__ldcg(x.ctl + K_WL0);
+    const int per = wcc_tile(nv);
     for (int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x; i - threadIdx.x < n;
          i += (int64_t)gridDim.x * kBlock) {
         const int32_t v = i < n ? x.roots[i] : 0, c = i < n ? r.aux[v] : 0;
-        const int32_t cs = c <= kLocalV ? c : 0;
+        const bool mid = c > kTileT && c <= kLocalV;
+        const int32_t cs = c <= kTileT ? c : 0;
         int32_t incl = cs;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -867,12 +879,18 @@ __global__ void __launch_bounds__(kBlock) k_wcc_alloc(Run<OffT> r, Ext<OffT> x) 
         unsigned long long at = 0;
         if (lane_id() == 31 && incl) at = atomicAdd(x.ctl + K_ALLOC, (unsigned long long)incl);
         at = __shfl_sync(kFull, at, 31);
-        const unsigned sm = __ballot_sync(kFull, cs > 0);
+        const unsigned sm = __ballot_sync(kFull, cs > 0 || mid);
         if (lane_id() == 0 && sm) atomicAdd(x.ctl + K_SMALL, (unsigned long long)__popc(sm));
         if (cs) {
             const int32_t b = (int32_t)at + incl - cs;
             r.aux2[v] = b;
             atomicMin(x.large[1] + b / per, b);
+        } else if (mid) {  // a tile of its own, from the back of the member list
+            const int32_t b = (int32_t)(nv - (int64_t)atomicAdd(x.ctl + K_MID_BACK, (unsigned long long)c)) - c;
+            r.aux2[v] = b;
+            const unsigned long long q = atomicAdd(x.ctl + K_MID, 1ull);
+            x.small[2 * q] = b;
+            x.small[2 * q + 1] = c;
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(r.counters + C_WCC, (unsigned long long)n);
@@ -911,20 +929,18 @@ __global__ void __launch_bounds__(kBlock) k_wcc_scatter(Run<OffT> r, Ext<OffT> x
 // or, where their edges overflow it, one by one; a WCC whose own edges
 // overflow it spills to the large path.  A serial Tarjan per WCC that was not
 // one SCC, by one thread, took 782 us for 8 WCCs of a 23-graph batch, and
-// 5,320 rings with chords 169 us a breadth-first level at a time; as tiles they
-// take about 350 and 80 us.
-using LocalTile = Tile<2 * kLocalV, 12288, 512>;
+// 5,320 rings with chords 169 us a breadth-first level at a time.
 
 template <typename OffT>
-__global__ void __launch_bounds__(LocalTile::kThreads) k_local_scc(Run<OffT> r, Ext<OffT> x) {
+__global__ void __launch_bounds__(TileSmem::kThreads) k_local_scc(Run<OffT> r, Ext<OffT> x) {
     pdl_wait();  // predecessor done, its writes visible
     pdl_trigger();
     if (__ldcg(x.ctl + K_TINY)) return;  // the residual was solved in one CTA
     extern __shared__ __align__(16) unsigned char tile_raw[];
-    using T = LocalTile;
+    using T = TileSmem;
     T &t = *reinterpret_cast<T *>(tile_raw);
     const int tid = threadIdx.x, lane = lane_id();
-    const int64_t total = (int64_t)__ldcg(x.ctl + K_ALLOC);
+    const int64_t total = (int64_t)__ldcg(x.ctl + K_ALLOC), mids = (int64_t)__ldcg(x.ctl + K_MID);
     const int per = wcc_tile((int64_t)__ldcg(x.ctl + K_WL0));
     const int64_t tiles = (total + per - 1) / per;
     const int32_t *first = x.large[1];
@@ -932,9 +948,12 @@ __global__ void __launch_bounds__(LocalTile::kThreads) k_local_scc(Run<OffT> r, 
     for (;;) {
         __syncthreads();  // the previous tile's readers are done
         if (tid == 0) {
-            const int64_t k = (int64_t)atomicAdd(x.ctl + K_LOCAL_NEXT, 1ull);
+            const int64_t w = (int64_t)atomicAdd(x.ctl + K_LOCAL_NEXT, 1ull), k = w - mids;
             int64_t a = 0, z = -1;
-            if (k < tiles) {
+            if (w < mids) {  // the larger ones first
+                a = x.small[2 * w];
+                z = a + x.small[2 * w + 1];
+            } else if (k < tiles) {
                 a = first[k];
                 z = total;
                 for (int64_t j = k + 1; j < tiles; ++j)
@@ -954,24 +973,25 @@ __global__ void __launch_bounds__(LocalTile::kThreads) k_local_scc(Run<OffT> r, 
             if (tid == 0) t.edges = 0;
             for (int i = tid; i < T::kV / 32; i += T::kThreads) t.dead[i] = 0u;
             __syncthreads();
-            int32_t v[T::kPer];
+            for (int i = tid; i < n; i += T::kThreads) t.f[i] = r.members[lo + i];
+            tile_sort(t, n);
             for (int u = 0; u < T::kPer && u * T::kThreads < n; ++u) {
                 const int i = u * T::kThreads + tid;
-                v[u] = i < n ? r.members[lo + i] : -1;
-                const int64_t e0 = v[u] >= 0 ? ld_off(r.fw_beg, v[u]) : 0, e1 = v[u] >= 0 ? ld_off(r.fw_beg, v[u] + 1) : 0;
+                const int32_t v = i < n ? t.orig[i] : -1;
+                const int64_t e0 = v >= 0 ? ld_off(r.fw_beg, v) : 0, e1 = v >= 0 ? ld_off(r.fw_beg, v + 1) : 0;
                 // the active neighbours: a lane reads a short list, the warp a long one
                 int32_t d = 0;
                 for (int64_t e = e0; e < min(e1, e0 + kLocalLane); e += 4) {
                     int32_t w[4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) w[q] = e + q < min(e1, e0 + kLocalLane) ? ld_adj(r.fw_adj, e + q) : v[u];
+                    for (int q = 0; q < 4; ++q) w[q] = e + q < min(e1, e0 + kLocalLane) ? ld_adj(r.fw_adj, e + q) : v;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) d += w[q] != v[u] && bitc(r.A, w[q]);
+                    for (int q = 0; q < 4; ++q) d += w[q] != v && bitc(r.A, w[q]);
                 }
                 for (unsigned g = __ballot_sync(kFull, e1 - e0 > kLocalLane); g; g &= g - 1) {
                     const int l = __ffs(g) - 1;
                     const int64_t le = __shfl_sync(kFull, e1, l);
-                    const int32_t lv = __shfl_sync(kFull, v[u], l);
+                    const int32_t lv = __shfl_sync(kFull, v, l);
                     int c = 0;
                     for (int64_t e = __shfl_sync(kFull, e0, l) + kLocalLane + lane; e < le; e += 32) {
                         const int32_t w = ld_adj(r.fw_adj, e);
@@ -989,10 +1009,7 @@ __global__ void __launch_bounds__(LocalTile::kThreads) k_local_scc(Run<OffT> r, 
                 int32_t at = 0;
                 if (lane == 31) at = atomicAdd(&t.edges, incl);
                 at = __shfl_sync(kFull, at, 31);
-                if (v[u] >= 0) {
-                    t.orig[i] = v[u];
-                    t.f[i] = i;
-                    t.b[i] = i;
+                if (v >= 0) {
                     t.off[i] = (uint16_t)min(at + incl - d, 0xffff);
                     t.len[i] = (uint16_t)min(d, 0xffff);
                 }
@@ -1014,14 +1031,15 @@ __global__ void __launch_bounds__(LocalTile::kThreads) k_local_scc(Run<OffT> r, 
             } else {
                 for (int u = 0; u < T::kPer && u * T::kThreads < n; ++u) {
                     const int i = u * T::kThreads + tid;
-                    const int64_t e0 = v[u] >= 0 ? ld_off(r.fw_beg, v[u]) : 0, e1 = v[u] >= 0 ? ld_off(r.fw_beg, v[u] + 1) : 0;
-                    int32_t p = v[u] >= 0 ? t.off[i] : 0;
+                    const int32_t v = i < n ? t.orig[i] : -1;
+                    const int64_t e0 = v >= 0 ? ld_off(r.fw_beg, v) : 0, e1 = v >= 0 ? ld_off(r.fw_beg, v + 1) : 0;
+                    int32_t p = v >= 0 ? t.off[i] : 0;
                     for (int64_t e = e0; e < min(e1, e0 + kLocalLane); e += 4) {
                         int32_t w[4], l[4];
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) w[q] = e + q < min(e1, e0 + kLocalLane) ? ld_adj(r.fw_adj, e + q) : v[u];
+                        for (int q = 0; q < 4; ++q) w[q] = e + q < min(e1, e0 + kLocalLane) ? ld_adj(r.fw_adj, e + q) : v;
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) l[q] = w[q] != v[u] && bitc(r.A, w[q]) ? r.cnt_in[w[q]] - lo : -1;
+                        for (int q = 0; q < 4; ++q) l[q] = w[q] != v && bitc(r.A, w[q]) ? t.f[r.cnt_in[w[q]] - lo] : -1;
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
                             if (l[q] >= 0 && ICHK(l[q] < n && p < T::kE, 14, ((long long)p << 32) | l[q])) t.adj[p++] = (uint16_t)l[q];
@@ -1029,13 +1047,13 @@ __global__ void __launch_bounds__(LocalTile::kThreads) k_local_scc(Run<OffT> r, 
                     for (unsigned g = __ballot_sync(kFull, e1 - e0 > kLocalLane); g; g &= g - 1) {
                         const int l = __ffs(g) - 1;
                         const int64_t le = __shfl_sync(kFull, e1, l);
-                        const int32_t lv = __shfl_sync(kFull, v[u], l);
+                        const int32_t lv = __shfl_sync(kFull, v, l);
                         int32_t lp = __shfl_sync(kFull, p, l);
                         for (int64_t e = __shfl_sync(kFull, e0, l) + kLocalLane; e < le; e += 32) {
                             const int32_t w = e + lane < le ? ld_adj(r.fw_adj, e + lane) : lv;
                             const bool in = w != lv && bitc(r.A, w);
                             const unsigned m = __ballot_sync(kFull, in);
-                            if (in) t.adj[lp + __popc(m & lanemask_lt())] = (uint16_t)(r.cnt_in[w] - lo);
+                            if (in) t.adj[lp + __popc(m & lanemask_lt())] = (uint16_t)t.f[r.cnt_in[w] - lo];
                             lp += __popc(m);
                         }
                     }

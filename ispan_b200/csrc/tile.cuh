@@ -7,7 +7,10 @@
 // atomicMin, b pulled by its owner, so the out-lists alone are enough; a
 // label also jumps to the label of its holder, so a ring takes about
 // log(length) passes.  Where f = b = p the vertex is in p's SCC; the others
-// go on, classed by (f, b), their lists pruned to their class.
+// go on, classed by (f, b), their lists pruned to their class.  The local ids
+// are the ranks of the original ids: where ids follow the edges, the lowest
+// label among the descendants (or ancestors) is the SCC's own, and two rounds
+// end what random labels split in half per round.
 //
 // What bounds it: shared-memory accesses at random addresses (about ten a
 // vertex and pass) and the passes' barriers: 8,192 vertices on 1,024 threads
@@ -28,17 +31,58 @@ struct Tile {
     int32_t start, count, edges;
 };
 
-// Solve the tile's n vertices (orig, the lists and f[i] = b[i] = i written,
-// dead cleared; the caller's threads need not have met since): labels,
+// Sort the tile's vertices by original id.  Before: f[i] the original id of
+// the i-th vertex; after: orig[j] the original ids in order, b[j] the place i
+// that each came from, f[i] the rank j of the i-th (padding left out).  A
+// bitonic sort over the next power of two.
+template <typename T>
+__device__ __forceinline__ void tile_sort(T &t, int n) {
+    int m = 32;
+    while (m < n) m <<= 1;
+    for (int i = threadIdx.x; i < m; i += T::kThreads) {
+        if (i >= n) t.f[i] = 0x7fffffff;
+        t.b[i] = i;
+    }
+    for (int k = 2; k <= m; k <<= 1)
+        for (int j = k >> 1; j; j >>= 1) {
+            __syncthreads();
+            for (int q = threadIdx.x; q < m / 2; q += T::kThreads) {
+                const int a = 2 * q - (q & (j - 1)), c = a + j;  // j apart, a's bit j clear
+                const int x = t.f[a], y = t.f[c];
+                if ((x > y) == ((a & k) == 0)) {
+                    t.f[a] = y;
+                    t.f[c] = x;
+                    const int z = t.b[a];
+                    t.b[a] = t.b[c];
+                    t.b[c] = z;
+                }
+            }
+        }
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += T::kThreads) t.orig[j] = t.f[j];
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += T::kThreads) t.f[t.b[j]] = j;
+    __syncthreads();
+}
+
+// Solve the tile's n vertices (orig and the lists written, dead cleared; the
+// caller's threads need not have met since): labels,
 // classes, histogram entries; the thread's vertices and SCCs are added to
 // done and sccs.  Ends with a barrier.
 template <typename T, typename RunT>
 __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &done, int64_t &sccs) {
     constexpr int kPer = T::kPer;
     const int tid = threadIdx.x;
+    __syncthreads();  // the lists' builders are done with f and b
     unsigned mine = 0;  // my vertices not solved yet
 #pragma unroll
     for (int u = 0; u < kPer; ++u) mine |= (u * T::kThreads + tid < n ? 1u : 0u) << u;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+        if ((mine >> u) & 1u) {
+            t.f[u * T::kThreads + tid] = u * T::kThreads + tid;
+            t.b[u * T::kThreads + tid] = u * T::kThreads + tid;
+        }
     for (int round = 0;; ++round) {
         if (round > n) {  // every round finds the SCC of each class's lowest label
             if (tid == 0) atomicCAS(r.err, 0, kErrOverflow);

@@ -1,5 +1,6 @@
 """The splitting, tile and labelling kernels of the large WCCs (resolve.cuh) on
-graphs whose residual is built to reach their edges: components one vertex
+graphs whose residual is built to reach their edges, and the cycles along near
+ids (cycles.cuh): components one vertex
 below, at and above the tile sizes, lists longer than a lane reads alone, a
 component too dense for a tile, duplicate edges and self-loops; exact labels
 against the oracle's Tarjan."""
@@ -60,11 +61,11 @@ def _blocks(sizes, dag, seed, scramble, chords=0.5, dense=0, join=True):
 # WCCs below, at and above the limit of the shared-memory path, tiles whose
 # edges overflow (solved WCC by WCC) and a WCC whose own do (spilled)
 SMALL = {
-    "limits": dict(sizes=[1023, 1024, 1025, 2, 3, 1] + [4] * 700, dag=0),
+    "limits": dict(sizes=[4095, 4096, 4097, 8192, 8193, 2, 3, 1] + [4] * 700, dag=0),
     "one tile": dict(sizes=[9, 5, 4], dag=0),
-    "dense": dict(sizes=[400] + [30] * 60, dag=0, dense=9000),
-    "overflow": dict(sizes=[500] + [600] * 4, dag=0, dense=14000),
-    "chords": dict(sizes=[100] * 30, dag=0, chords=9.0),
+    "dense": dict(sizes=[100] * 12, dag=0, chords=400.0),
+    "overflow": dict(sizes=[100] * 12, dag=0, chords=500.0),
+    "chords": dict(sizes=[1000] * 30, dag=0, chords=9.0),
 }
 
 CASES = {
@@ -75,6 +76,55 @@ CASES = {
     "long ring": dict(sizes=[70000, 5, 5], dag=30, chords=0.0),
     "nothing joins": dict(sizes=[3000] * 30, dag=0),
 }
+
+
+def _renumber(csr, order):
+    """csr with vertex order[i] renamed i."""
+    to = np.empty(csr.V, np.int64)
+    to[order] = np.arange(csr.V)
+    src = np.repeat(np.arange(csr.V), np.diff(csr.fw_beg))
+    return _csr(csr.V, to[src], to[csr.fw_adj])
+
+
+# ids along the rings: rings in topological order, in the reverse of it and in
+# random order (where only the peel of the contracted rings ends them), rings
+# with chords, one longer than the longest walk, a closing edge that is not
+# the nearest in-edge, and ids without locality inside some blocks
+NEAR = {
+    "order": dict(sizes=[300] * 60 + [2, 3, 900, 1], dag=30000, chords=0.0),
+    "chords": dict(sizes=[40] * 300, dag=20000, chords=0.3),
+    "pairs": dict(sizes=[2] * 4000, dag=12000, chords=0.0),
+    "long": dict(sizes=[20000, 30, 16384, 16385, 500], dag=40000, chords=0.0),
+    "few": dict(sizes=[900] * 6, dag=11000, chords=0.02),
+}
+
+
+@pytest.mark.parametrize("name", list(NEAR))
+@pytest.mark.parametrize("ids", ["up", "down", "blocks", "mixed"])
+def test_cycles_along_ids(name, ids):
+    import oracle
+    from ispan_b200 import Context
+    c = NEAR[name]
+    csr = _blocks(seed=len(name), scramble=False, **c)
+    rng = np.random.default_rng(7)
+    n = sum(c["sizes"])
+    order = np.arange(csr.V)
+    if ids == "down":
+        order[:n] = order[:n][::-1]
+    elif ids == "blocks":
+        off = np.concatenate([[0], np.cumsum(c["sizes"])])
+        perm = rng.permutation(len(c["sizes"]))
+        order[:n] = np.concatenate([np.arange(off[k], off[k + 1]) for k in perm])
+    elif ids == "mixed":
+        order[:n // 3] = rng.permutation(n // 3)
+    csr = _renumber(csr, order)
+    exact = oracle.tarjan(csr)
+    with Context(csr.V, csr.E) as ctx:
+        for graph in (True, False):
+            labels, st = ctx.run_csr(csr, histogram=True, use_graph=graph)
+            assert np.array_equal(labels, exact)
+            assert st["histogram"] == oracle.histogram(exact)
+            assert st["scc_count"] == len(np.unique(exact))
 
 
 @pytest.mark.parametrize("name", list(SMALL))
@@ -88,7 +138,7 @@ def test_small_wccs(name, graph):
         labels, st = ctx.run_csr(csr, histogram=True, use_graph=graph)
     assert np.array_equal(labels, exact)
     assert st["histogram"] == oracle.histogram(exact)
-    assert st["local_wcc"] == st["n_wcc"] - (name == "limits") - (name == "overflow")
+    assert st["local_wcc"] == st["n_wcc"] - {"limits": 1, "overflow": 12}.get(name, 0)
 
 
 @pytest.mark.parametrize("name", list(CASES))
