@@ -33,6 +33,7 @@
 #include "resolve.cuh"
 #include "tiny.cuh"
 #include "cycles.cuh"
+#include "small.cuh"
 #include "lane.h"
 #include "stages.cuh"
 
@@ -183,6 +184,7 @@ struct ispan_ctx {
     // captures of the conditional parts of the graph, the inner one second
     cudaStream_t stream_if[2] = {nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    bool small_fits = false;    // k_small's cluster can be resident
     int g_coop_w = 0;           // offset width the coop grids were computed for
 
     // CUDA graph cache
@@ -458,6 +460,32 @@ static cudaError_t launch_k(bool pdl, void (*k)(P...), int64_t grid, int block, 
     return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// k_small: one cluster
+static cudaLaunchConfig_t small_config(cudaLaunchAttribute (&at)[2], bool pdl, cudaStream_t s) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3(kSmallCtas);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = sizeof(SmallSmem);
+    cfg.stream = s;
+    memset(at, 0, sizeof at);
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kSmallCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 2 : 1;
+    return cfg;
+}
+
+template <typename... P, typename... A>
+static cudaError_t launch_small(bool pdl, void (*k)(P...), cudaStream_t s, A... args) {
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = small_config(at, pdl, s);
+    return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 template <typename Kern, typename... Args>
 static cudaError_t launch_coop(Kern k, int grid, cudaStream_t s, Args... args) {
     void *ptrs[] = {(void *)&args...};
@@ -553,6 +581,14 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
         rd.nseg = r.nseg;
         PK((k_reset), std::min<int64_t>(G, 4 * c->nsm), 256, rd);
     }
+    // k_small where its maps fit: measured at R-MAT scale 16 104 us a call against 150 with the stage kernels, at
+    // scale 10 72 against 115.  Stage times, exact statistics and the tiny kernel's tuning need the stage kernels.
+    const bool small = c->small_fits && r.V <= kSmallV && r.E <= kSmallE && !times && !(r.flags & ISPAN_F_EXACT_STATS) &&
+                       c->tuning.tiny_residual <= 0;
+    if (small) {  // all up to the first peel in one cluster
+        if ((e = launch_small(pdl_ok && prev_plain, k_small<OffT>, s, r, x))) return e;
+        prev_plain = false;
+    } else {
     PK((k_trim1_first<OffT>), G, kBlock, r, x);
     EV(1);
     const int gseed = (int)std::max<int64_t>(1, (r.nseg + 1023) / 1024);
@@ -605,6 +641,7 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     prev_plain = false;
     if (r.flags & ISPAN_F_EXACT_STATS) PK((k_list_degrees<OffT>), G, kBlock, r, r.wl[1], x.ctl + K_WL1, C_Q2_N, C_Q2_XDEG);
     EV(5);
+    }
     if (gates) {
         if ((e = if_begin(s, c->stream_if[0], x.gate_left, &if_left))) return e;
         s = c->stream_if[0];
@@ -719,11 +756,18 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     prev_plain = false;
     if (gates) {
         if ((e = if_end(c->stream_if[0], s, if_large))) return e;
-        if ((e = if_end(c->stream, c->stream_if[0], if_left))) return e;
-        s = c->stream;
+        s = c->stream_if[0];
+        if (!small) {
+            if ((e = if_end(c->stream, s, if_left))) return e;
+            s = c->stream;
+        }
     }
     EV(11);
     PK((k_finalize<OffT>), G, kBlock, r, x);
+    if (gates && small) {  // (k_small finalises what it ends itself)
+        if ((e = if_end(c->stream, s, if_left))) return e;
+        s = c->stream;
+    }
     EV(12);
 #undef EV
 #undef LK
@@ -750,6 +794,15 @@ static int coop_setup(ispan_ctx *c) {
     c->g_coop[3] = coop_grid(k_color<OffT>, nsm, kBlock);
     c->g_coop[4] = std::min(coop_grid(k_split, nsm, kBlock), coop_grid(k_resolve, nsm, kBlock));
     CK(cudaFuncSetAttribute(k_local_scc<OffT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
+    CK(cudaFuncSetAttribute(k_small<OffT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallSmem)));
+    CK(cudaFuncSetAttribute(k_small<OffT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    {  // (a part of a GPU may have no 16 SMs side by side)
+        cudaLaunchAttribute at[2];
+        const cudaLaunchConfig_t cfg = small_config(at, false, nullptr);
+        int n = 0;
+        c->small_fits = cudaOccupancyMaxActiveClusters(&n, k_small<OffT>, &cfg) == cudaSuccess && n > 0;
+        (void)cudaGetLastError();
+    }
     CK(cudaFuncSetAttribute(k_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
     c->g_coop[5] = coop_grid(k_cycles<OffT>, nsm, kBlock);
     c->g_coop[6] = coop_grid(k_super<OffT>, nsm, kBlock);

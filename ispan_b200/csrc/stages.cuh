@@ -30,6 +30,7 @@ enum Ctl64 {
     K_TICKET0 = K_RES_WORK + 12,   // CTAs done with the first peel,
     K_TICKET1,                     // with k_local_scc (see set_gate)
     K_MID, K_MID_BACK,             // WCCs with a tile of their own, their vertices
+    K_SMALL_DONE,                  // 1: k_small wrote all labels; the finalisation returns at once
     K_CYC_ON, K_CYC_N, K_CYC_MEM, K_CYC_LEFT,  // cycles.cuh: cycles were looked for (2: most edges lead down),
                                    // vertices on those found, places taken, vertices on none,
     K_SUP_Q, K_SUP_LEFT = K_SUP_Q + 3,  // vertices to peel (3 slots), vertices left
@@ -1649,6 +1650,7 @@ template <typename OffT>
 __global__ void __launch_bounds__(kBlock) k_finalize(Run<OffT> r, Ext<OffT> x) {
     pdl_wait();  // predecessor done, its writes visible
     pdl_trigger();
+    if (__ldcg(x.ctl + K_SMALL_DONE)) return;
     constexpr int U = 4;
     const int lane = lane_id();
     const int64_t gw = ((int64_t)blockIdx.x * kBlock + threadIdx.x) >> 5;
