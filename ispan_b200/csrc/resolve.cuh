@@ -111,6 +111,17 @@ __device__ __forceinline__ typename ResVal<K>::T res_warp_join(typename ResVal<K
     return x;
 }
 
+// The entry of v's list whose original id is nearest to its own (v if none).
+__device__ __forceinline__ int32_t res_near(const ResBufs &m, int d, int32_t v) {
+    const int32_t mine = m.old[v];
+    int32_t at = v, near = 0x7fffffff;
+    for (int32_t k = m.beg[d][v], e = m.end[d][v]; k < e; ++k) {
+        const int32_t w = m.adj[d][k], far = abs(m.old[w] - mine);
+        if (far < near) { near = far; at = w; }
+    }
+    return at;
+}
+
 // One dense step of direction d for four vertices of a lane (v < 0: none):
 // their list ranges, then their entries four by four, then the entries'
 // values, each group of loads in flight together; a list's entries beyond
@@ -177,6 +188,47 @@ __device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int3
             ch |= 1u << u;
         }
     return ch;
+}
+
+// The same for one vertex of a lane (v < 0: none), over its link too: the link
+// then jumps to its target's, which is read before the target's value (that
+// covers all between).  again: the link starts anew.
+template <int K>
+__device__ __forceinline__ bool res_pull_linked(const ResBufs &m, int d, int32_t v, uint32_t *link, bool again) {
+    using T = typename ResVal<K>::T;
+    T *val = reinterpret_cast<T *>(m.val[d]);
+    const int32_t *adj = m.adj[d];
+    int32_t b = 0, e = 0;
+    T own = 0, nw = 0;
+    if (v >= 0) {
+        b = m.beg[d][v];
+        e = m.end[d][v];
+        const uint32_t far = __ldcg(link + v), to = __ldcg(link + far);
+        own = __ldcg(val + v);
+        nw = res_join<K>(own, __ldcg(val + far));
+        if constexpr (K == R_MIN) nw = min(nw, __ldcg(val + own));
+        __stcg(link + v, again ? (uint32_t)res_near(m, d, v) : to);
+    }
+    const int32_t c = min(e, b + kResLane);
+    for (; b < c; b += 4) {
+        int32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[q] = b + q < c ? adj[b + q] : v;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) nw = res_join<K>(nw, __ldcg(val + w[q]));
+    }
+    b = min(b, e);
+    for (unsigned g = __ballot_sync(kFull, b < e); g; g &= g - 1) {
+        const int l = __ffs(g) - 1;
+        const int32_t lb = __shfl_sync(kFull, b, l), le = __shfl_sync(kFull, e, l);
+        T acc = (T)__shfl_sync(kFull, nw, l);
+        for (int32_t k = lb + lane_id(); k < le; k += 32) acc = res_join<K>(acc, __ldcg(val + adj[k]));
+        acc = res_warp_join<K>(acc);
+        if (lane_id() == l) nw = acc;
+    }
+    if (nw == own) return false;
+    __stcg(val + v, nw);
+    return true;
 }
 
 // The listed vertices of a warp (ent valid where have) push: a forward value
@@ -254,6 +306,14 @@ constexpr int kResTail = 1024;
 constexpr int kResTailLevels = 256;  // levels in CTA 0 before the grid meets again
 constexpr int kResBudget = 1024;
 constexpr int kResHops = 64;
+// Few vertices take dense passes to the end, over links too (see Tile): a pass
+// costs what a level does, ~9 us, and the links end rings of a thousand hops
+// in tens of passes.  (What 97 separate graphs left after the tiles, 44,000
+// vertices: 4.5 ms of levels, 0.66 with links.)  Many vertices have no links:
+// two more gathers in a pass of about three, measured 7.6 ms -> 10.7 on a web
+// graph of 1.1 M vertices here.
+constexpr int64_t kResLinkN = 1 << 18;
+constexpr int kResAgain = 10;          // passes after which the links start anew: 2^10 hops
 struct ResSmem {
     int64_t sum[kWarps];
     uint32_t q[2][2 * kResTail];
@@ -261,23 +321,45 @@ struct ResSmem {
 };
 template <int K>
 __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &m, unsigned long long *chg,
-                                           unsigned long long *qc, const int32_t *list, int64_t n, int dirs, int &s,
+                                           unsigned long long *qc, const unsigned long long *x_large, const int32_t *list, int64_t n, int dirs, int &s,
                                            ResSmem &sm) {
     const int64_t gt = (int64_t)blockIdx.x * kBlock + threadIdx.x;
     const int64_t nt = (int64_t)gridDim.x * kBlock;
     bool dense = true;
     int64_t prev = n * 2, nq = 0;
     int cur = 0, levels = 0, hops = 0;
+    // few vertices: links, and dense passes to the end
+    const bool linked = n <= kResLinkN;
+    uint32_t *link[2] = {nullptr, nullptr};
+    if (linked) {
+        const int64_t all = (int64_t)__ldcg(x_large);
+        for (int d = 0; d < 2; ++d) {
+            if (!((dirs >> d) & 1)) continue;
+            link[d] = K == R_MIN ? m.val[d] + all : m.val[d ^ 1];  // (masks spread one way at a time)
+            for (int64_t i = gt; i < n; i += nt) {
+                const int32_t v = list ? list[i] : (int32_t)i;
+                link[d][v] = (uint32_t)res_near(m, d, v);
+            }
+        }
+        if (!grid_sync(r.gsync, r.err)) return 0;
+    }
     for (int64_t guard = 0; guard <= 128 * (r.V + 2); ++guard) {  // every pass lowers a value or sets a bit
         const int s1 = s == 2 ? 0 : s + 1;
         if (blockIdx.x == 0 && threadIdx.x == 0) { chg[s1] = 0ull; qc[s1] = 0ull; }
         if (K != R_MIN && levels > kResBudget) return 2;
         if (dense) {
             // few changes in the last pass: the vertices that change now are listed
-            const bool listing = prev <= n / kResSparse;
+            const bool listing = prev <= n / kResSparse && !linked;
             int changed = 0;
+            if (linked)
+                for (int64_t i = gt; i - threadIdx.x < n; i += nt) {
+                    const int32_t v = i < n ? (list ? list[i] : (int32_t)i) : -1;
+                    for (int d = 0; d < 2; ++d)
+                        if ((dirs >> d) & 1)
+                            changed += res_pull_linked<K>(m, d, v, link[d], levels % kResAgain == kResAgain - 1);
+                }
             const int64_t gw = gt >> 5, nw = nt >> 5;
-            for (int64_t i0 = gw * (32 * kResU); i0 < n; i0 += nw * (32 * kResU)) {
+            for (int64_t i0 = gw * (32 * kResU); i0 < n && !linked; i0 += nw * (32 * kResU)) {
                 int32_t v[kResU];
 #pragma unroll
                 for (int u = 0; u < kResU; ++u) {
@@ -526,8 +608,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
             else v16[v] = pivot ? (unsigned short)(1u << (mix32(h) & 15u)) : (unsigned short)0;
         }
         if (!grid_sync(r.gsync, r.err)) return;
-        const int ok = wide ? res_spread<R_OR64>(r, m, chg, qc, list, nl, 1 << d, s, sm)
-                            : res_spread<R_OR16>(r, m, chg, qc, list, nl, 1 << d, s, sm);
+        const int ok = wide ? res_spread<R_OR64>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm)
+                            : res_spread<R_OR16>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm);
         if (ok == 0) return;
         if (ok == 2) {  // these masks say nothing; the labelling rounds take what no tile does
             if (gt == 0) x.ctl[K_RES_STOP] = 1ull;
@@ -740,7 +822,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
             m.size[v] = 0;
         }
         if (!grid_sync(r.gsync, r.err)) return;
-        if (res_spread<R_MIN>(r, m, chg, qc, list, nl, 3, s, sm) != 1) return;
+        if (res_spread<R_MIN>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 3, s, sm) != 1) return;
         for (int64_t i = gt; i < nl; i += nt) {
             const int32_t v = list[i];
             const uint32_t f = __ldcg(m.val[0] + v);

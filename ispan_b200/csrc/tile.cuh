@@ -12,18 +12,33 @@
 // label among the descendants (or ancestors) is the SCC's own, and two rounds
 // end what random labels split in half per round.
 //
-// What bounds it: shared-memory accesses at random addresses (about ten a
+// That jump helps one direction: where ids ascend along a ring, the lowest
+// descendant's label comes back one edge a pass.  So every vertex also keeps
+// a link to a descendant and one to an ancestor (first the neighbour nearest by
+// id), joins their labels and jumps to their links: after k passes a link
+// spans 2^k edges and the label is the lowest along them.  A label that
+// arrives later somewhere under a long link is missed by it, so the links
+// start anew every kTileAgain passes.
+//
+// What bounds it: shared-memory accesses at random addresses (about fifteen a
 // vertex and pass) and the passes' barriers: 8,192 vertices on 1,024 threads
-// take about 5 us a pass, 300-450 us a tile.
+// take about 6 us a pass.  Pieces of time-ordered DAGs of rings (2,000 to 7,500
+// vertices): 75 to 1,280 passes without the links, up to 4 ms a tile; with
+// them 17 to 28 passes, 50-230 us.
 #pragma once
 #include "common.cuh"
 
 namespace ispan {
 
+constexpr int kTileAgain = 10;  // passes after which the links start anew: 2^10 hops
+
 template <int V_, int E_, int THREADS>
 struct Tile {
     static constexpr int kV = V_, kE = E_, kThreads = THREADS, kPer = V_ / THREADS;
-    int32_t orig[V_];        // original ids
+    union {
+        int32_t orig[V_];      // original ids; while solving:
+        uint16_t link[2][V_];  // an ancestor, a descendant
+    };
     int32_t f[V_], b[V_];
     uint16_t off[V_], len[V_];
     uint16_t adj[E_];
@@ -65,6 +80,19 @@ __device__ __forceinline__ void tile_sort(T &t, int n) {
     __syncthreads();
 }
 
+// i's links anew: the descendant nearest by id, and i as that one's ancestor
+// (of several, any).
+template <typename T>
+__device__ __forceinline__ void tile_link(T &t, int i) {
+    int near = 0xffff, at = i;
+    for (int k = t.off[i], z = k + t.len[i]; k < z; ++k) {
+        const int w = t.adj[k], far = abs(w - i);
+        if (far < near && far) { near = far; at = w; }
+    }
+    t.link[1][i] = (uint16_t)at;
+    t.link[0][at] = (uint16_t)i;
+}
+
 // Solve the tile's n vertices (orig and the lists written, dead cleared; the
 // caller's threads need not have met since): labels,
 // classes, histogram entries; the thread's vertices and SCCs are added to
@@ -73,22 +101,31 @@ template <typename T, typename RunT>
 __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &done, int64_t &sccs) {
     constexpr int kPer = T::kPer;
     const int tid = threadIdx.x;
-    __syncthreads();  // the lists' builders are done with f and b
     unsigned mine = 0;  // my vertices not solved yet
 #pragma unroll
     for (int u = 0; u < kPer; ++u) mine |= (u * T::kThreads + tid < n ? 1u : 0u) << u;
+    int32_t orig[kPer];
 #pragma unroll
-    for (int u = 0; u < kPer; ++u)
-        if ((mine >> u) & 1u) {
-            t.f[u * T::kThreads + tid] = u * T::kThreads + tid;
-            t.b[u * T::kThreads + tid] = u * T::kThreads + tid;
-        }
+    for (int u = 0; u < kPer; ++u) orig[u] = (mine >> u) & 1u ? t.orig[u * T::kThreads + tid] : 0;
+    __syncthreads();  // the lists' builders are done with f and b, and orig is read
     for (int round = 0;; ++round) {
         if (round > n) {  // every round finds the SCC of each class's lowest label
             if (tid == 0) atomicCAS(r.err, 0, kErrOverflow);
             break;
         }
-        // (the barrier of the first test: lists and labels are in place)
+        // labels and links: the descendant nearest by id, and the reverse
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            if (!((mine >> u) & 1u)) continue;
+            const int i = u * T::kThreads + tid;
+            t.f[i] = t.b[i] = i;
+            t.link[0][i] = (uint16_t)i;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kPer; ++u)
+            if ((mine >> u) & 1u) tile_link(t, u * T::kThreads + tid);
+        // (the barrier of the first test: lists, labels and links are in place)
         // after k passes a label has come k edges far, so n passes are enough
         int pass = 0;
         for (int ch = 1; __syncthreads_or(ch); ++pass) {
@@ -103,8 +140,12 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
                 const int i = u * T::kThreads + tid;
                 volatile int32_t *f = t.f, *b = t.b;
                 const int32_t f0 = f[i], b0 = b[i];
-                const int32_t fv = min(f0, f[f0]);
-                int32_t bv = min(b0, b[b0]);
+                // the link's link before its label: that then covers all between them
+                volatile uint16_t *anc = t.link[0], *des = t.link[1];
+                const int la = anc[i], ld = des[i];
+                const uint16_t la2 = anc[la], ld2 = des[ld];
+                const int32_t fv = min(min(f0, f[f0]), f[la]);
+                int32_t bv = min(min(b0, b[b0]), b[ld]);
                 const int o = t.off[i], z = o + t.len[i];
                 for (int k = o; k < z; ++k) {
                     const int w = t.adj[k];
@@ -113,6 +154,12 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
                 }
                 if (fv < f0) { atomicMin(&t.f[i], fv); ch = 1; }
                 if (bv < b0) { b[i] = bv; ch = 1; }
+                if (pass % kTileAgain != kTileAgain - 1) {
+                    anc[i] = la2;
+                    des[i] = ld2;
+                } else {
+                    tile_link(t, i);
+                }
             }
         }
         // solved: f = b = p.  A solved p gathers its SCC's lowest
@@ -134,7 +181,7 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
             const int i = u * T::kThreads + tid;
             if ((sol >> u) & 1u) atomicOr(&t.dead[i >> 5], 1u << (i & 31));
             if ((roots >> u) & 1u) {
-                t.f[i] = t.orig[i];
+                t.f[i] = orig[u];
                 t.b[i] = 1;
             }
         }
@@ -144,7 +191,7 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
             const int i = u * T::kThreads + tid;
             if (((sol & ~roots) >> u) & 1u) {
                 const int p = t.f[i];
-                atomicMin(&t.f[p], t.orig[i]);
+                atomicMin(&t.f[p], orig[u]);
                 atomicAdd(&t.b[p], 1);
             }
         }
@@ -154,7 +201,7 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
             const int i = u * T::kThreads + tid;
             if (!((sol >> u) & 1u)) continue;
             const bool root = (roots >> u) & 1u;
-            const int32_t lab = root ? t.f[i] : t.f[t.f[i]], ov = t.orig[i];
+            const int32_t lab = root ? t.f[i] : t.f[t.f[i]], ov = orig[u];
             r.label[ov] = lab;
             r.cls[ov] = CLS_MICE;
             clear_bit(r.A, ov);
@@ -180,13 +227,6 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
             t.len[i] = (uint16_t)(q - o);
         }
         if (!__syncthreads_or(mine != 0u)) break;
-#pragma unroll
-        for (int u = 0; u < kPer; ++u)
-            if ((mine >> u) & 1u) {
-                const int i = u * T::kThreads + tid;
-                t.f[i] = i;
-                t.b[i] = i;
-            }
     }
 }
 

@@ -155,3 +155,22 @@ def test_exact_labels(name, scramble):
             assert st["histogram"] == oracle.histogram(exact)
             assert st["scc_count"] == len(np.unique(exact))
             assert st["n_mice_vertices"] >= 65536  # the large-WCC path ran
+
+
+# a component left to splitting and labelling just at and just above the size
+# up to which values spread over links, with ids along its ring (chords make
+# it several rings), against them and at random
+@pytest.mark.parametrize("size", [262144, 262145])
+@pytest.mark.parametrize("ids", ["up", "down", "mixed"])
+def test_links(size, ids):
+    import oracle
+    from ispan_b200 import Context
+    csr = _blocks([size, 3, 500], dag=200, seed=3, scramble=ids == "mixed", chords=0.02)
+    if ids == "down":
+        csr = _renumber(csr, np.arange(csr.V)[::-1])
+    exact = oracle.tarjan(csr)
+    with Context(csr.V, csr.E) as ctx:
+        for graph in (True, False):
+            labels, st = ctx.run_csr(csr, histogram=True, use_graph=graph)
+            assert np.array_equal(labels, exact)
+            assert st["histogram"] == oracle.histogram(exact)
