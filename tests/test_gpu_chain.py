@@ -1,0 +1,56 @@
+"""Searches along rings and paths of consecutive ids (the look-ahead of the
+asynchronous mode, bfs.cuh): stretches one id shorter than, as long as and
+longer than a warp looks ahead, up and down, past hubs and to both ends of the
+id range; exact labels against the oracle's Tarjan."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _stretches(length, down, hubs, V=80000, tail=3000, seed=1):
+    """One ring over stretches of `length` consecutive ids in random order, two
+    paths hanging off it (one in, one out), short side edges; hubs: every 97th
+    vertex of the ring has 40 more edges ahead of its own stretch."""
+    rng = np.random.default_rng(seed)
+    n = V - 2 * tail
+    ids = np.arange(tail, tail + n)
+    starts = np.arange(0, n, length)
+    order = rng.permutation(len(starts))
+    ring = np.concatenate([ids[starts[k]:starts[k] + length] for k in order])
+    if down:
+        ring = ring[::-1]
+    S, D = [ring], [np.roll(ring, -1)]
+    out, into = np.arange(tail), np.arange(V - tail, V)  # both ends of the id range
+    for p in (out, into):
+        S.append(p[:-1])
+        D.append(p[1:])
+    S += [ring[5:6], into[-1:]]
+    D += [out[:1], ring[9:10]]
+    if hubs:
+        h = np.repeat(ring[::97], 40)
+        S.append(h)
+        D.append(out[rng.integers(0, tail, len(h))])
+    S, D = np.concatenate(S), np.concatenate(D)
+    o = rng.permutation(len(S))
+    return V, S[o], D[o]
+
+
+@pytest.mark.parametrize("length", [1, 2, 14, 15, 16, 17, 31, 33, 74000])
+@pytest.mark.parametrize("down", [False, True])
+@pytest.mark.parametrize("hubs", [False, True])
+def test_stretches(length, down, hubs):
+    import oracle
+    from ispan_b200 import Context
+    from ispan_b200.graphs import from_edges
+    V, s, d = _stretches(length, down, hubs)
+    csr = from_edges(V, np.stack([s, d], 1))
+    exact = oracle.tarjan(csr)
+    with Context(csr.V, csr.E) as ctx:
+        for pair in (1, -1):
+            ctx.set_tuning(pair_searches=pair)
+            for graph in (True, False):
+                labels, st = ctx.run_csr(csr, use_graph=graph)
+                assert np.array_equal(labels, exact)
+                assert st["giant_size"] == 74000
+                assert st["fw_size"] == 74000 + 2999  # (the last of the path out is trimmed)
