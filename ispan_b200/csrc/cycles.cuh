@@ -32,8 +32,8 @@
 // graphs with permuted ids) both kernels return at once.
 //
 // A batch of 512 graphs (82 M vertices, 42 M residual), one B200: colouring
-// 250 ms of a run's 298; k_cycles 6.5 ms (list reads 2.0, the rest latency of
-// walks) and k_super 3.5 ms (one edge pass, a scan, the labels), a run 46 ms.
+// 250 ms of a run's 298; k_cycles 3.0 ms (list reads 2.0, the rest latency of
+// walks) and k_super 3.5 ms (one edge pass, a scan, the labels), a run 37 ms.
 // With the peel alone instead of the spans 32 ms and 18 ms for what rings in
 // pieces kept from it.
 #pragma once
@@ -112,6 +112,21 @@ __device__ __forceinline__ void choose_single(const Run<OffT> &r, const CycBufs 
 __device__ __forceinline__ int32_t cyc_next(const CycBufs &b, int32_t node) {
     const unsigned long long k = __ldcg(b.key + node);
     return k == ~0ull ? node : cyc_node(b, (int32_t)(k & 0x7fffffffu));
+}
+
+// How many hops a walk over nodes goes from u along consecutive ids in steps
+// of dir, all over single vertices: a warp looks at 32 of them at once.  (Hop by
+// hop, three dependent reads each, the walks of rings of up to 1,000 took most
+// of this kernel: on 97 separate graphs 3.1 ms before, 0.31 so; on 512 graphs in
+// one batch 6.5 and 3.0.)
+template <typename OffT>
+__device__ __forceinline__ int cyc_run(const Run<OffT> &r, const CycBufs &b, int32_t u, int dir) {
+    const int64_t x = (int64_t)u + (int64_t)lane_id() * dir;
+    const bool single = x >= 0 && x < r.V && bitc(r.A, x) && !bitv(r.D, x);
+    const unsigned long long k = single ? __ldcg(b.key + x) : ~0ull;
+    const bool hop = k != ~0ull && (int64_t)(k & 0x7fffffffu) == x + dir;
+    const unsigned s = __ballot_sync(kFull, single);
+    return __ffs(~(__ballot_sync(kFull, hop) & (s >> 1))) - 1;
 }
 
 // skip: pointers mostly lead to the id next to their own; runs of such
@@ -332,35 +347,73 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
         }
         if (!grid_sync(r.gsync, r.err)) return;
         // nodes of several vertices choose single ones only, so every cycle
-        // has a single vertex: its lowest one walks it
-        for (int64_t i = gt; i < ns1; i += nt) {
-            const int32_t v = b.single[i];
-            if (bitv(r.D, v)) continue;
-            int32_t u = cyc_next(b, v), low = v, mark = u;
-            int len = 1;
-            // (a mark renewed at powers of two: met again, the walk is in a cycle without v)
-            while (u != v && len < kCycMax && !(u < v && __ldcg(b.size + u) == 1)) {
-                low = min(low, u);
-                u = cyc_next(b, u);
-                if (u == mark) break;
-                if ((++len & (len - 1)) == 0) mark = u;
-            }
-            if (u != v || len < 2) continue;  // a lower single vertex, another cycle, too long, or no choice
-            int all = 0, fresh = 0;
-            int32_t w = v;
-            for (int k = 0; k < len; ++k) {
-                const int32_t nw = cyc_next(b, w);  // (read before w's rep changes)
-                const int sz = __ldcg(b.size + w);
-                all += sz;
-                if (sz == 1) {
-                    ++fresh;
-                    set_bit(r.D, w);
+        // has a single vertex: its lowest one walks it, a warp a walk
+        for (int64_t i = gt; i - lane_id() < ns1; i += nt) {
+            const int32_t mine = i < ns1 ? b.single[i] : 0;
+            int32_t first = mine;
+            if (i < ns1 && !bitv(r.D, mine)) first = cyc_next(b, mine);
+            for (unsigned g = __ballot_sync(kFull, first != mine && !(first < mine && __ldcg(b.size + first) == 1)); g;
+                 g &= g - 1) {
+                const int l = __ffs(g) - 1;
+                const int32_t v = __shfl_sync(kFull, mine, l);
+                int32_t u = __shfl_sync(kFull, first, l), low = v, mark = u;
+                int len = 1, dir = -1, renew = 2;
+                bool found = false;
+                // (a mark renewed at powers of two: met again, the walk is in a cycle without v)
+                while (len < kCycMax && !(u < v && __ldcg(b.size + u) == 1)) {
+                    low = min(low, u);
+                    const int c = cyc_run(r, b, u, dir);
+                    if (c > 0) {
+                        const int64_t jv = ((int64_t)v - u) * dir, jm = ((int64_t)mark - u) * dir;
+                        if (jv >= 1 && jv <= c) {
+                            len += (int)jv;
+                            found = true;
+                            break;
+                        }
+                        if (jm >= 1 && jm <= c) break;
+                        u += c * dir;
+                        len += c;
+                    } else {
+                        const int32_t nu = cyc_next(b, u);
+                        if (abs(nu - u) == 1) dir = nu - u;
+                        u = nu;
+                        if (u == mark) break;
+                        ++len;
+                        if (u == v) {
+                            found = true;
+                            break;
+                        }
+                    }
+                    if (len >= renew) {
+                        mark = u;
+                        renew = 2 * len;
+                    }
                 }
-                if (w != low) b.rep[w] = low;
-                w = nw;
+                if (!found) continue;  // a lower single vertex, another cycle, too long, or no choice
+                int all = 0, fresh = 0;
+                int32_t w = v;
+                for (int k = 0; k < len;) {
+                    const int c = min(cyc_run(r, b, w, dir), len - k);
+                    const int32_t nw = c > 0 ? w + c * dir : cyc_next(b, w);  // (read before w's rep changes)
+                    const int sz = c > 0 ? c : __ldcg(b.size + w);
+                    __syncwarp();
+                    if (lane_id() < max(c, 1)) {
+                        const int32_t y = w + lane_id() * dir;
+                        if (c > 0 || sz == 1) set_bit(r.D, y);
+                        if (y != low) b.rep[y] = low;
+                    }
+                    __syncwarp();
+                    all += sz;
+                    fresh += c > 0 ? c : sz == 1;
+                    if (c == 0 && abs(nw - w) == 1) dir = nw - w;
+                    k += max(c, 1);
+                    w = nw;
+                }
+                if (lane_id() == 0) {
+                    b.size[low] = all;
+                    atomicAdd(x.ctl + K_CYC_N, (unsigned long long)fresh);
+                }
             }
-            b.size[low] = all;
-            atomicAdd(x.ctl + K_CYC_N, (unsigned long long)fresh);
         }
         if (!grid_sync(r.gsync, r.err)) return;
         const int64_t now = (int64_t)__ldcg(x.ctl + K_CYC_N);
