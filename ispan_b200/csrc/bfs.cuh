@@ -384,13 +384,14 @@ struct AsyncSmem {
 
 constexpr int kAsyncFlush = kLQ / 2;  // a CTA's local frontier above this is work for the whole grid
 
-// A frontier vertex v of the async mode, by a warp that looks ahead along ids:
-// lane k reads the list of v + k, lane 15 + k that of v - k, all at once.  As
-// long as each of them leads to the next the whole stretch is reached, and
-// every lane expands the vertex it claims.  On a ring or path of consecutive
-// ids one level goes 15 vertices far; a level is four dependent reads (offsets,
-// list, visit map, degrees, ~3 us) whatever it reaches.  Only where the CTA's
-// frontier is at most kChainN vertices: a wider one keeps a lane per vertex.
+// A frontier vertex v of the async mode, by a warp that looks ahead along ids.
+// If v leads to v + 1 (v - 1), lane k reads the list of v + k (lane 15 + k that
+// of v - k), all at once.  As long as each of them leads to the next the whole
+// stretch is reached, and every lane expands the vertex it claims.  On a ring
+// or path of consecutive ids one level goes 15 vertices far; a level is five
+// dependent reads (offsets, list, visit map, degrees, ~3 us) whatever it
+// reaches.  Only where the CTA's frontier is at most kChainN vertices: a wider
+// one keeps a lane per vertex.
 // (97 separate graphs, rings of up to 1,000: the async rounds of the two
 // searches 1,570 and 880 us by single steps, 850 and 130 so.)
 constexpr int kChainN = 2 * kWarps;
@@ -399,34 +400,32 @@ __device__ __forceinline__ void async_chain(const Run<OffT> &r, const BfsDir<Off
                                             int64_t *qen, int32_t *qcn, unsigned long long *pk_next, int64_t &nvis,
                                             int64_t &msum_next, Expand expand) {
     const int lane = lane_id();
-    const int step = lane < 16 ? 1 : -1;
-    const int64_t x = lane < 16 ? (int64_t)v + lane : (int64_t)v - (lane - 15);
-    const bool have = x >= 0 && x < r.V && (lane == 0 || bit(d.R, x));
-    int64_t x0 = 0, x1 = 0;
-    if (have) {
-        x0 = ld_off(d.xbeg, x);
-        x1 = ld_off(d.xbeg, x + 1);
-    }
-    bool next = false, down = false;  // x leads to x + step; v to v - 1
-    for (int64_t e = x0, z = min(x1, x0 + (int64_t)kAsyncDeg); e < z; e += 4) {
-        int32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[q] = e + q < z ? ld_adj(d.xadj, e + q) : -2;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            next |= w[q] == x + step;
-            down |= w[q] == v - 1;
+    const int64_t v0 = ld_off(d.xbeg, v), v1 = ld_off(d.xbeg, v + 1);
+    const int32_t w0 = v0 + lane < v1 ? ld_adj(d.xadj, v0 + lane) : -2;
+    const unsigned up = __ballot_sync(kFull, w0 == v + 1), dn = __ballot_sync(kFull, w0 == v - 1);
+    if (up | dn) {
+        const int step = lane < 16 ? 1 : -1;
+        const int64_t x = lane < 16 ? (int64_t)v + lane : (int64_t)v - (lane - 15);
+        const bool have = (lane < 16 ? up && lane > 0 : dn != 0) && x >= 0 && x < r.V && bit(d.R, x);
+        int64_t x0 = 0, x1 = 0;
+        if (have) {
+            x0 = ld_off(d.xbeg, x);
+            x1 = ld_off(d.xbeg, x + 1);
         }
-    }
-    const unsigned nx = __ballot_sync(kFull, next), hv = __ballot_sync(kFull, have);
-    const unsigned dn = __ballot_sync(kFull, down) & 1u;
-    // bit j: the (j + 1)-th vertex that way is reached from the j-th
-    const unsigned up_ok = nx & 0x7fffu & (hv >> 1), dn_ok = (dn | ((nx >> 16) << 1)) & (hv >> 16);
-    const int n_up = __ffs(~up_ok) - 1, n_dn = __ffs(~dn_ok) - 1;
-    if (lane == 0) {
-        expand(x0, x1);  // whatever its degree
-    } else if (lane < 16 ? lane <= n_up : lane - 15 <= n_dn) {
-        if (!bitv(d.Vm, x) && set_bit(d.Vm, (int32_t)x)) {
+        bool next = false;  // x leads to x + step
+        for (int64_t e = x0, z = min(x1, x0 + (int64_t)kAsyncDeg); e < z; e += 4) {
+            int32_t w[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w[q] = e + q < z ? ld_adj(d.xadj, e + q) : -2;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) next |= w[q] == x + step;
+        }
+        const unsigned nx = __ballot_sync(kFull, next), hv = __ballot_sync(kFull, have);
+        // bit j: the (j + 1)-th vertex that way is reached from the j-th
+        const unsigned up_ok = ((nx & 0x7fffu) | (up ? 1u : 0u)) & (hv >> 1) & 0x7fffu;
+        const unsigned dn_ok = ((dn ? 1u : 0u) | ((nx >> 16) << 1)) & (hv >> 16);
+        const int n_up = __ffs(~up_ok) - 1, n_dn = __ffs(~dn_ok) - 1;
+        if (have && (lane < 16 ? lane <= n_up : lane - 15 <= n_dn) && !bitv(d.Vm, x) && set_bit(d.Vm, (int32_t)x)) {
             ++nvis;
             if (x1 - x0 <= r.async_deg) {
                 expand(x0, x1);
@@ -435,7 +434,9 @@ __device__ __forceinline__ void async_chain(const Run<OffT> &r, const BfsDir<Off
                 msum_next += x1 - x0;
             }
         }
+        __syncwarp();
     }
+    for (int64_t e = v0 + lane; e < v1; e += 32) expand(e, e + 1);  // whatever its degree
     __syncwarp();
 }
 
@@ -539,15 +540,26 @@ __device__ __forceinline__ void rebuild_queue(const Run<OffT> &r, const BfsDir<O
     for (int64_t wb = w_begin * 32; wb < r.W; wb += w_stride * 32) {
         const int64_t my = wb + lane;
         uint32_t nw = my < r.W ? (__ldcg(d.Vm + my) & ~__ldcg(r.P + my)) : 0u;
-        unsigned has = __ballot_sync(kFull, nw != 0);
-        while (has) {
-            int l = __ffs(has) - 1;
-            has &= has - 1;
-            uint32_t m = __shfl_sync(kFull, nw, l);
-            bool me = (m >> lane) & 1u;
-            int64_t v = (wb + l) * 32 + lane;
-            int64_t dg = me ? d.xdeg(v) : 0;
-            q_append(me, (int32_t)v, dg, r.qv[nx], r.qe[nx], r.qchunk[nx], pk, r.V);
+        // the set bits of the 32 words, 32 at a time: one reservation in the
+        // queue for them, not one per word
+        int incl = __popc(nw);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int total = __shfl_sync(kFull, incl, 31), excl = incl - __popc(nw);
+        for (int j0 = 0; j0 < total; j0 += 32) {
+            const int j = j0 + lane;
+            int l = 0;  // the word: the number of lanes whose prefix is at most j
+#pragma unroll
+            for (int st = 16; st; st >>= 1)
+                if (__shfl_sync(kFull, incl, l + st - 1) <= j) l += st;
+            const bool me = j < total;
+            uint32_t m = __shfl_sync(kFull, nw, l & 31);
+            for (int k = j - __shfl_sync(kFull, excl, l & 31); me && k > 0; --k) m &= m - 1;
+            const int64_t v = (wb + l) * 32 + __ffs(m) - 1;
+            q_append(me, (int32_t)v, me ? d.xdeg(v) : 0, r.qv[nx], r.qe[nx], r.qchunk[nx], pk, r.V);
         }
     }
 }
@@ -579,7 +591,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Run<OffT> r, BfsCtl *ctl) {
     const int64_t n_total = (int64_t)(over_a ? r.counters[C_ACTIVE0] : r.counters[C_FW_SIZE]);
     int level = 0, mode = M_TD;
     bool left_bu = false;  // like the reference, a search never returns to bottom-up
-    int64_t total_vis = 0;
+    int64_t total_vis = 0, nf_last = 0;
     // small frontiers go to the async mode; larger ones stay top-down
     const int64_t av = r.async_v, ae = r.async_e;
     auto small = [av, ae](int64_t qc, int64_t qe) { return qc <= av && qe <= ae; };
@@ -639,7 +651,13 @@ __global__ void __launch_bounds__(kBlock, 2) k_bfs(Run<OffT> r, BfsCtl *ctl) {
         const int64_t qcn = (int64_t)(pn & kCountMask), qen = (int64_t)(pn >> kCountBits);
         if (mode == M_BU) {
             if (nf == 0) { mode = M_DONE; break; }
-            if (nf < n_total / max(r.beta, 1) || level > r.gamma) {
+            // a level reads the lists of all that is unreached; what ebbs away
+            // far below that is pushed.  (Two levels that found 790,000 and
+            // 42,000 of 60 M vertices of a batch, 40 M of them not to be
+            // reached: 1.7 ms each; the second pushed: 0.12.)
+            const bool ebbs = 4 * nf < n_total - total_vis && 4 * nf < nf_last;
+            nf_last = nf;
+            if (nf < n_total / max(r.beta, 1) || level > r.gamma || ebbs) {
                 // leave bottom-up for good: queue the vertices found this level
                 left_bu = true;
                 rebuild_queue<OffT, DIR>(r, d, level & 1, r.qpk + (level % 3), gwarp, nwarps);

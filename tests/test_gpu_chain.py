@@ -54,3 +54,32 @@ def test_stretches(length, down, hubs):
                 assert np.array_equal(labels, exact)
                 assert st["giant_size"] == 74000
                 assert st["fw_size"] == 74000 + 2999  # (the last of the path out is trimmed)
+
+
+@pytest.mark.parametrize("second", [1400, 3000, 14999])
+def test_ebbing_search(second):
+    """A bottom-up level that found few beside what stays unreached hands them
+    to the top-down queue (from both dense and sparse words of the visit map)."""
+    import oracle
+    from ispan_b200 import Context
+    from ispan_b200.graphs import from_edges
+    leaves, third, pairs = 60000, 200, 100000
+    leaf = 1 + np.arange(leaves)
+    two = 1 + leaves + np.arange(second)
+    three = 1 + leaves + second + np.arange(third)
+    rest = 1 + leaves + second + third + np.arange(2 * pairs)
+    V = 1 + leaves + second + third + 2 * pairs
+    up = [(np.zeros(leaves, int), leaf), (leaf[::4][:second], two), (two[:third], three), (rest[::2], rest[1::2])]
+    S = np.concatenate([x for a, b in up for x in (a, b)])
+    D = np.concatenate([x for a, b in up for x in (b, a)])
+    p = np.arange(V)
+    p[leaves:] = leaves + np.random.default_rng(2).permutation(V - leaves)
+    csr = from_edges(V, np.stack([p[S], p[D]], 1))
+    exact = oracle.tarjan(csr)
+    with Context(csr.V, csr.E) as ctx:
+        for pair in (1, -1):
+            ctx.set_tuning(pair_searches=pair)
+            for graph in (True, False):
+                labels, st = ctx.run_csr(csr, use_graph=graph)
+                assert np.array_equal(labels, exact)
+                assert st["giant_size"] == st["fw_size"] == 1 + leaves + second + third
