@@ -1,26 +1,23 @@
-// compact.cuh -- the compact graph the colouring of large WCCs runs on.
+// compact.cuh -- the compact graph on which the large WCCs are split and solved
+// (resolve.cuh).
 //
-// The colouring rounds (k_color, stages.cuh) work on the vertices of the
-// large WCCs only: on web-shaped graphs ~15 % of the vertices, with a quarter
-// of their edges leading outside them (to the giant SCC, the trimmed
-// sources and sinks).  On the input graph every edge check reads a colour
-// word indexed over the whole vertex range and rejects the outside
-// neighbours by their class; the offsets and adjacency are read over the
-// whole CSR.  Here, before the rounds start, those vertices get dense ids
-// 0..n-1 (their order in the large-WCC list, i.e. about the input order) and
-// their edges among themselves are copied into a CSR of those ids, in the
-// context's scratch that is free at this point:
+// Those vertices are ~15 % of a web-shaped graph, with a quarter of their
+// edges leading outside them (to the giant SCC, the trimmed sources and
+// sinks).  On the input graph every edge check would read a word indexed over
+// the whole vertex range.  Here they get dense ids 0..n-1 (their order in the
+// large-WCC list, i.e. about the input order) and their edges among themselves
+// are copied into a CSR of those ids, in the context's scratch that is free at
+// this point:
 //   compact id -> original id   x.small      (int32, n)
 //   original id -> compact id   r.cnt_out    (int32, valid where A is set)
 //   out/in degrees              r.members, x.roots
 //   offsets (int32)             r.qe[1] viewed as int32: out at [0, n], in at [V+1, V+1+n]
 //   adjacency (int32)           r.wl[0..1] (out), r.members..x.roots (in, written once the
 //                               degrees there are scanned); each pair is one block of 2 V
-// so the random accesses of the rounds fall on n colour words instead of V,
-// and no edge check lands on a vertex outside.  The graph is built only when
+// so the random accesses of the rounds fall on n words instead of V, and no
+// edge check lands on a vertex outside.  The graph is built only when
 // each direction's edges fit the adjacency arrays (at most V entries, int32
-// offsets); otherwise K_CMP_OK stays 0 and the colouring runs on the input
-// graph.  Membership is the active map A: at this point exactly the vertices
+// offsets); otherwise K_CMP_OK stays 0 and k_color runs on the input graph.  Membership is the active map A: at this point exactly the vertices
 // of the large WCCs are active.  The fill kernel reads only the offsets, so
 // the in-adjacency may overwrite the degree arrays.
 #pragma once

@@ -2,16 +2,19 @@
 // the stage launch sequence (captured once into a CUDA graph and replayed),
 // and the extern "C" boundary declared in include/ispan_b200.h.
 //
-// Stage sequence (reference src/scc_core.cpp:144-1070, same order):
+// Stage sequence (reference src/scc_core.cpp:144-1070, same order; k_small
+// takes all up to the first peel of a small graph):
 //   trim-1-first + pivot      k_trim1_first, k_seed
 //   elephant FW / BW          k_bfs<.,0>, k_bfs<.,1>   (persistent, cooperative)
 //   giant, residual           k_giant_residual
 //   trim-1 peel (fixpoint)    k_trim1                  (persistent, cooperative)
 //   trim-2, trim-3            k_trim2, k_trim3
 //   trim-1 peel again         k_trim1
+//   cycles along near ids     k_cycles                 (persistent, cooperative)
 //   WCC                       k_wcc_init/hook/compress/giant/hook/flatten/alloc/scatter
-//   mice: small WCCs          k_local_scc              (shared-memory Tarjan)
-//   mice: large WCCs          k_color                  (persistent, cooperative)
+//   mice: small WCCs          k_local_scc              (shared-memory tiles)
+//   mice: large WCCs          k_super, k_cmp_*, k_split + k_tiles, k_resolve (persistent, cooperative);
+//                             k_color where there is no compact graph
 //   canonical labels          k_finalize
 // Every kernel reads its work sizes from device memory, so the whole sequence
 // is enqueued without a host round trip and the host synchronises once.

@@ -34,7 +34,7 @@
 // MB, a pass took 1.3 ms, with 32-bit ones 0.53).  In the tails a level's
 // latency counts.  Web-shaped graphs, colouring stage before and now, one
 // B200: 7 M vertices (1.1 M here) 10.0 and 5.3 ms, 140 M vertices (21 M
-// here) 244 and 97 ms.
+// here) 244 and 85 ms.
 #pragma once
 #include "compact.cuh"
 #include "tile.cuh"
@@ -52,7 +52,8 @@ constexpr int64_t kResFew = 16;        // fewer vertices left than 1 / 16: no mo
 constexpr int64_t kResWideN = 6 << 20;
 constexpr int64_t kResNarrowN = 32 << 20;
 constexpr int64_t kResSparse = 16;     // a pass that changed at most 1 / 16 of the vertices ends the dense passes
-                                       // (a listed vertex costs ~0.2 ns to push, a dense pass ~0.015-0.025 ns a vertex)
+                                       // (a listed vertex costs ~0.17 ns to push, a dense pass ~0.01-0.017 ns a vertex);
+                                       // more listed ones than that begin them again
 constexpr uint32_t kResHash = 0x07ffffffu;  // class word while splitting: 27 bits of hash, 5 bits of log2 |WCC|
 constexpr uint32_t kResDead = 0xffffffffu;  // class word of a vertex whose SCC is known
 
@@ -293,7 +294,8 @@ __device__ __forceinline__ void res_push(const ResBufs &m, bool have, uint32_t e
 
 // Spread the values of the listed vertices (list null: all of [0, n)) to
 // the fixpoint in the directions of `dirs` (bit 0 forward, bit 1 backward).
-// s: the rotating counter slot.  Returns 1; 0 if a grid barrier failed; 2 if
+// s: the rotating counter slot; seeded: the vertices that hold a value are
+// listed already (q[0], their number in the slot).  Returns 1; 0 if a grid barrier failed; 2 if
 // it gave up, which only masks do, after about kResBudget levels: on long
 // paths without shortcuts they come one edge far per level, where labels jump
 // (after kResHops levels the labels take dense passes again).
@@ -322,7 +324,7 @@ struct ResSmem {
 template <int K>
 __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &m, unsigned long long *chg,
                                            unsigned long long *qc, const unsigned long long *x_large, const int32_t *list, int64_t n, int dirs, int &s,
-                                           ResSmem &sm) {
+                                           ResSmem &sm, bool seeded) {
     const int64_t gt = (int64_t)blockIdx.x * kBlock + threadIdx.x;
     const int64_t nt = (int64_t)gridDim.x * kBlock;
     bool dense = true;
@@ -342,6 +344,11 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
             }
         }
         if (!grid_sync(r.gsync, r.err)) return 0;
+    }
+    if (seeded) {
+        nq = (int64_t)__ldcg(qc + s);
+        s = s == 2 ? 0 : s + 1;
+        dense = linked || nq > n / kResSparse || nq > m.cap_q;
     }
     for (int64_t guard = 0; guard <= 128 * (r.V + 2); ++guard) {  // every pass lowers a value or sets a bit
         const int s1 = s == 2 ? 0 : s + 1;
@@ -371,15 +378,22 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
                     const unsigned ch = res_pull<K>(m, d, v);
                     changed += __popc(ch);
                     if (!listing) continue;
+                    unsigned g[kResU];
+                    int tot = 0;
 #pragma unroll
                     for (int u = 0; u < kResU; ++u) {
-                        const bool me = (ch >> u) & 1u;
-                        const unsigned g = __ballot_sync(kFull, me);
-                        if (!g) continue;
-                        unsigned long long at = 0;
-                        if (lane_id() == 0) at = atomicAdd(qc + s, (unsigned long long)__popc(g));
-                        at = __shfl_sync(kFull, at, 0) + __popc(g & lanemask_lt());
-                        if (me && (int64_t)at < m.cap_q) m.q[0][at] = (uint32_t)v[u] | ((uint32_t)d << 31);
+                        g[u] = __ballot_sync(kFull, (ch >> u) & 1u);
+                        tot += __popc(g[u]);
+                    }
+                    if (!tot) continue;
+                    unsigned long long at = 0;
+                    if (lane_id() == 0) at = atomicAdd(qc + s, (unsigned long long)tot);
+                    at = __shfl_sync(kFull, at, 0);
+#pragma unroll
+                    for (int u = 0; u < kResU; ++u) {
+                        const unsigned long long to = at + __popc(g[u] & lanemask_lt());
+                        if (((ch >> u) & 1u) && (int64_t)to < m.cap_q) m.q[0][to] = (uint32_t)v[u] | ((uint32_t)d << 31);
+                        at += __popc(g[u]);
                     }
                 }
             }
@@ -459,26 +473,28 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
         if (nq == 0) return 1;
         // a wide level, or entries that did not fit: dense passes again
         // (they see every vertex, so nothing unlisted is lost)
-        if (nq > n / 8 || nq > m.cap_q || (K == R_MIN && hops > kResHops)) { dense = true; prev = n * 2; }
+        if (nq > n / kResSparse || nq > m.cap_q || (K == R_MIN && hops > kResHops)) { dense = true; prev = n * 2; }
     }
     if (threadIdx.x == 0) atomicCAS(r.err, 0, kErrOverflow);
     return 0;
 }
 
-// Drop the list entries that lead out of their vertex's class.  A warp takes
+// Drop the list entries that lead out of their vertex's class (cls(v): its
+// class, or what now tells it from the others of its old one).  A warp takes
 // a group of 32 consecutive vertices, whose lists lie back to back (the
 // build writes them so and pruning keeps it), reads the group's entries 32
 // at a time, coalesced, and packs the kept ones to the group's front with
 // one ballot per step; each lane counts what its vertex keeps.  (A thread
 // per vertex storing its own kept entries took 6.6 ms for 2 x 65 M entries
 // of 21 M vertices, this form 1.8 ms.)
-__device__ __forceinline__ void res_prune(const ResBufs &m, int d, int64_t v0, int64_t n) {
+template <typename Cls>
+__device__ __forceinline__ void res_prune(const ResBufs &m, int d, int64_t v0, int64_t n, Cls cls) {
     const int lane = lane_id();
     const int64_t v = v0 + lane;
     const bool have = v < n;
     int32_t *adj = m.adj[d];
     const int32_t b0 = have ? m.beg[d][v] : 0, e0 = have ? m.end[d][v] : 0;
-    const uint32_t c = have ? m.cls[v] : kResDead;
+    const uint32_t c = have ? cls((int32_t)v) : kResDead;
     const int32_t len = e0 - b0;
     int32_t incl = len;
 #pragma unroll
@@ -497,7 +513,7 @@ __device__ __forceinline__ void res_prune(const ResBufs &m, int d, int64_t v0, i
             if (__shfl_sync(kFull, incl, o + st - 1) <= k) o += st;
         const uint32_t co = __shfl_sync(kFull, c, o & 31);
         const int32_t w = k < total ? __ldcg(adj + base + k) : -1;
-        const bool keep = w >= 0 && __ldcg(m.cls + w) == co;
+        const bool keep = w >= 0 && cls(w) == co;
         const unsigned g = __ballot_sync(kFull, keep);
         if (keep) __stcg(adj + base + out + __popc(g & lanemask_lt()), w);
         out += __popc(g);
@@ -519,8 +535,9 @@ __device__ __forceinline__ void res_prune(const ResBufs &m, int d, int64_t v0, i
 
 // The same for one vertex, where few of a group are left: its kept entries
 // move to the front of its own list.
-__device__ __forceinline__ void res_prune_one(const ResBufs &m, int32_t v) {
-    const uint32_t c = m.cls[v];
+template <typename Cls>
+__device__ __forceinline__ void res_prune_one(const ResBufs &m, int32_t v, Cls cls) {
+    const uint32_t c = cls(v);
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
         const int32_t b = m.beg[d][v], e = m.end[d][v];
@@ -532,7 +549,7 @@ __device__ __forceinline__ void res_prune_one(const ResBufs &m, int32_t v) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) u[q] = k + q < e ? __ldcg(adj + k + q) : -1;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) cu[q] = u[q] >= 0 ? __ldcg(m.cls + u[q]) : ~c;
+            for (int q = 0; q < 4; ++q) cu[q] = u[q] >= 0 ? cls(u[q]) : ~c;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
                 if (cu[q] == c) {
@@ -599,6 +616,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
         const int d = k & 1;
         unsigned long long *v64 = reinterpret_cast<unsigned long long *>(m.val[d]);
         unsigned short *v16 = reinterpret_cast<unsigned short *>(m.val[d]);
+        if (gt == 0) { chg[s == 2 ? 0 : s + 1] = 0ull; qc[s == 2 ? 0 : s + 1] = 0ull; }
         for (int64_t i = gt; i < nl; i += nt) {
             const int32_t v = list ? list[i] : (int32_t)i;
             const uint32_t h = mix32((uint32_t)v * 16u + (uint32_t)(4 * it + k) + 1u);
@@ -606,10 +624,14 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
             const bool pivot = (h >> (32 - shift)) == 0u;
             if (wide) v64[v] = pivot ? 1ull << (mix32(h) & 63u) : 0ull;
             else v16[v] = pivot ? (unsigned short)(1u << (mix32(h) & 15u)) : (unsigned short)0;
+            if (pivot) {
+                const unsigned long long at = atomicAdd(qc + s, 1ull);
+                if ((int64_t)at < m.cap_q) m.q[0][at] = (uint32_t)v | ((uint32_t)d << 31);
+            }
         }
         if (!grid_sync(r.gsync, r.err)) return;
-        const int ok = wide ? res_spread<R_OR64>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm)
-                            : res_spread<R_OR16>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm);
+        const int ok = wide ? res_spread<R_OR64>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm, true)
+                            : res_spread<R_OR16>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm, true);
         if (ok == 0) return;
         if (ok == 2) {  // these masks say nothing; the labelling rounds take what no tile does
             if (gt == 0) x.ctl[K_RES_STOP] = 1ull;
@@ -621,14 +643,23 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
             const unsigned long long y = wide ? __ldcg(v64 + v) : (unsigned long long)__ldcg(v16 + v);
             m.cls[v] = (mix32(c ^ mix32((uint32_t)y ^ mix32((uint32_t)(y >> 32)))) & kResHash) | (c & ~kResHash);
         }
-        if (!grid_sync(r.gsync, r.err)) return;
-        if (4 * nl >= n)
-            for (int64_t g = gt >> 5; g * 32 < n; g += nt >> 5) {
-                res_prune(m, 0, g * 32, n);
-                res_prune(m, 1, g * 32, n);
-            }
-        else
-            for (int64_t i = gt; i < nl; i += nt) res_prune_one(m, list[i]);
+        const auto prune = [&](auto cls) {
+            if (4 * nl >= n)
+                for (int64_t g = gt >> 5; g * 32 < n; g += nt >> 5) {
+                    res_prune(m, 0, g * 32, n, cls);
+                    res_prune(m, 1, g * 32, n, cls);
+                }
+            else
+                for (int64_t i = gt; i < nl; i += nt) res_prune_one(m, list[i], cls);
+        };
+        // an entry led to the same class before, so 16-bit masks tell where it
+        // leads now: half the words to gather (21 M vertices, 84 MB of class words: 1.4-1.9 ms a round)
+        if (wide) {
+            if (!grid_sync(r.gsync, r.err)) return;
+            prune([&](int32_t w) { return __ldcg(m.cls + w); });
+        } else {
+            prune([&](int32_t w) { return (uint32_t)__ldcg(v16 + w); });
+        }
         if (!grid_sync(r.gsync, r.err)) return;
         ++rounds;
     }
@@ -822,7 +853,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
             m.size[v] = 0;
         }
         if (!grid_sync(r.gsync, r.err)) return;
-        if (res_spread<R_MIN>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 3, s, sm) != 1) return;
+        if (res_spread<R_MIN>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 3, s, sm, false) != 1) return;
         for (int64_t i = gt; i < nl; i += nt) {
             const int32_t v = list[i];
             const uint32_t f = __ldcg(m.val[0] + v);
@@ -885,7 +916,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
         }
         list = next;
         nl = nn;
-        for (int64_t i = gt; i < nl; i += nt) res_prune_one(m, list[i]);
+        for (int64_t i = gt; i < nl; i += nt) res_prune_one(m, list[i], [&](int32_t w) { return __ldcg(m.cls + w); });
         if (!grid_sync(r.gsync, r.err)) return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) r.counters[C_COLOR_ROUNDS] = (unsigned long long)rounds;

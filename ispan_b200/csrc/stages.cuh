@@ -19,7 +19,7 @@ namespace ispan {
 enum Ctl64 {
     K_WL0 = 0, K_WL1, K_CQ0, K_CQ1, K_CQ2, K_ROOTS, K_SMALL, K_LARGE, K_ALLOC, K_LARGE2,
     K_SPILL, K_MICE_SCC, K_LOCAL_NEXT, K_MINPRIO0, K_MINPRIO1, K_CAND,
-    K_CMP_OK, K_CMP_EF, K_CMP_EB,  // compact colouring graph: built (1), its edge counts
+    K_CMP_OK, K_CMP_EF, K_CMP_EB,  // compact graph: built (1), its edge counts
     K_WCC_GIANT,                   // (root << 32) | 1 when one WCC holds half the root sample
     K_TINY,                        // 1: k_tiny_residual solved the residual; later stages return at once
     K_RES_CHG,                     // k_resolve (resolve.cuh): values changed in a pass (3 slots),
