@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kThreads) k_cross_pairs(const OffT *__restrict
     for (int64_t u = warp; u < V; u += nwarps) {
         const int64_t e0 = (int64_t)beg[u], e1 = (int64_t)beg[u + 1];
         const uint32_t lu = (uint32_t)__ldg(label + u);
-        for (int64_t e = e0; e - lane < e1; e += 32) {
+        for (int64_t e = e0; e < e1; e += 32) {  // (the same steps in every lane: lane 0 reserves for all)
             bool cross = false;
             unsigned long long key = 0;
             if (e + lane < e1) {

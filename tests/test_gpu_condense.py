@@ -53,3 +53,20 @@ def test_condensation_matches_oracle(make):
     want = expected_pairs(csr, exact)
     assert np.array_equal(got, want.reshape(-1, 2))
     assert is_acyclic(got, np.unique(exact))
+
+
+def test_every_pair_of_long_lists():
+    """Lists shorter than, as long as and longer than one and two steps of a
+    warp, every entry a pair of its own: all of them, in every call."""
+    import torch
+    lens = np.array([0, 1, 2, 30, 31, 32, 33, 34, 62, 63, 64, 65, 66, 95, 96, 97, 130] * 40)
+    n, V = len(lens), len(lens) + 131
+    src = np.repeat(np.arange(n), lens)
+    dst = n + np.concatenate([np.arange(k) for k in lens])
+    csr = G.from_edges(V, np.stack([src, dst], 1))  # a DAG: every vertex its own SCC
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    lab = torch.arange(V, dtype=torch.int32, device="cuda")
+    want = expected_pairs(csr, np.arange(V))
+    assert len(want) == lens.sum()
+    for _ in range(5):
+        assert np.array_equal(condensation(t(csr.fw_beg), t(csr.fw_adj), lab), want)
