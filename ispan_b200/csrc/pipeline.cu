@@ -179,6 +179,7 @@ struct ispan_ctx {
 
     // copies from ordinary host memory (see copy_staged)
     char *h_stage = nullptr;  // pinned, kStageThreads x 2 pieces
+    bool stage_again = false;  // a call that could have staged came before
     bool stage_failed = false;
     cudaEvent_t ev_stage[2 * kStageThreads] = {};  // piece copied
 
@@ -1265,6 +1266,12 @@ static bool copy_staged(ispan_ctx *c, const HostCopy *cp, int n, cudaError_t &er
     }
     if (total < kStageMin || c->stage_failed || std::thread::hardware_concurrency() < 4) return false;
     if (!c->h_stage) {
+        // a context's first such call does without: pinning the pieces can cost
+        // it more (5-60 ms) than it gains
+        if (!c->stage_again) {
+            c->stage_again = true;
+            return false;
+        }
         bool ok = cudaMallocHost(&c->h_stage, 2 * kStageThreads * kStagePiece) == cudaSuccess;
         if (!ok) c->h_stage = nullptr;
         for (cudaEvent_t &e : c->ev_stage)
