@@ -314,7 +314,13 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
             const unsigned long long k = __ldcg(b.key + h);
             const int32_t u = (int32_t)(unsigned)k;
             left = k == ~0ull || (h <= u ? v < h || v > u : v < u || v > h);
-            if (!left) {
+            if (left && __ldcg(b.size + v) > 1) {
+                // a cycle's minimum whose pointer leads to the id after it: the
+                // mark of the ascending run it begins names the place of entry
+                // behind it (rep[v] is v already)
+                left = false;
+                set_bit(r.D, v);
+            } else if (!left) {
                 b.rep[v] = (int32_t)(k >> 32);
                 set_bit(r.D, v);
             }

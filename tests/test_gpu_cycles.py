@@ -1,0 +1,72 @@
+"""The contraction of cycles along near ids (cycles.cuh) on graphs large enough
+to reach it (32,768 residual vertices in WCCs above the tiles' size): labels,
+the size histogram and the SCC count against the oracle's Tarjan.  A node's
+size is read from the histogram, and by the peel of the nodes as the length of
+its slice of the node order."""
+import numpy as np
+import pytest
+
+from test_gpu_resolve import _csr
+
+pytestmark = pytest.mark.gpu
+
+CYC_MIN = 32768  # residual vertices from which cycles are looked for
+
+
+def _gadgets(count, size, edges, dag, seed, order):
+    """`count` copies of a gadget (edges among ids [0, size)), joined into one
+    WCC by a line and `dag` random edges from earlier to later copies, beside a
+    hub graph (the pivot's SCC).  The copies' ids: in the order of the DAG
+    ("up"), against it ("down"), or at random ("blocks", where no span of
+    descending edges ends a node and the peel runs)."""
+    rng = np.random.default_rng(seed)
+    e = np.array(edges)
+    place = {"up": np.arange(count), "down": np.arange(count)[::-1], "blocks": rng.permutation(count)}[order]
+    base = place * size
+    x, y = rng.integers(0, count, dag), rng.integers(0, count, dag)
+    x, y = np.minimum(x, y), np.maximum(x, y)
+    keep = x < y
+    x, y = x[keep], y[keep]
+    S = [(base[:, None] + e[None, :, 0]).ravel(), base[:-1], base[x] + rng.integers(0, size, len(x))]
+    D = [(base[:, None] + e[None, :, 1]).ravel(), base[1:], base[y] + rng.integers(0, size, len(y))]
+    n, h = count * size, 1200
+    S += [np.full(h, n), n + 1 + np.arange(h)]
+    D += [n + 1 + np.arange(h), np.full(h, n)]
+    return _csr(n + h + 1, np.concatenate(S), np.concatenate(D))
+
+
+def _check(csr, runs=3):
+    import oracle
+    from ispan_b200 import Context
+    exact = oracle.tarjan(csr)
+    hist = oracle.histogram(exact)
+    with Context(csr.V, csr.E) as ctx:
+        for k in range(runs):
+            labels, st = ctx.run_csr(csr, histogram=True, use_graph=k % 3 != 2)
+            assert np.array_equal(labels, exact)
+            assert st["histogram"] == hist
+            assert st["scc_count"] == len(np.unique(exact))
+            assert st["n_mice_vertices"] >= CYC_MIN  # cycles were looked for
+
+
+def _ring_down(lo, hi):
+    """A ring whose edges lead to the id before: its minimum's nearest
+    in-neighbour is the id after it."""
+    return [(i + 1, i) for i in range(lo, hi)] + [(lo, hi)]
+
+
+# a descending ring whose minimum lies on a way of single vertices back to the
+# ring (they are joined to it, and its size counts), and two such rings joined
+# both ways through their minima
+ASCENDING = {
+    "way": (56, _ring_down(5, 55) + [(i, i + 1) for i in range(4)] + [(4, 7), (6, 0)]),
+    "minima": (80, _ring_down(0, 39) + _ring_down(40, 79) + [(0, 40), (40, 0)]),
+    "two": (60, _ring_down(2, 57) + [(0, 1), (1, 0), (1, 2), (2, 58), (58, 59), (59, 2)]),
+}
+
+
+@pytest.mark.parametrize("name", list(ASCENDING))
+@pytest.mark.parametrize("order", ["up", "down", "blocks"])
+def test_minimum_that_leads_up(name, order):
+    size, edges = ASCENDING[name]
+    _check(_gadgets(1500, size, edges, dag=9000, seed=len(name), order=order))
