@@ -50,8 +50,9 @@ constexpr int kSuperTail = 1024;    // a round of the peel of at most this many 
 constexpr int kSuperTailRounds = 256;
 
 struct CycBufs {
-    int32_t *par;     // [V] nearest in-neighbour
-    int32_t *skip;    // [V] where the run of consecutive ids that the pointers follow from here ends
+    int32_t *par;     // [V] nearest in-neighbour; later, at a single vertex, the lowest id of the cycle it found
+    int32_t *skip;    // [V] where the run of consecutive ids that the pointers follow from here ends; later, at a
+                      // single vertex, the number of nodes of the cycle it found (0: none)
     int32_t *rep;     // [V] minimum of the vertex's node
     int32_t *size;    // [V] at a node's minimum: its vertices
     unsigned long long *key;  // [V] first: at a run's end, the walk through it (minimum, entry); then, at a node's
@@ -352,11 +353,17 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
             if (!bitv(r.D, v)) choose_single(r, b, v);
         }
         if (!grid_sync(r.gsync, r.err)) return;
-        // nodes of several vertices choose single ones only, so every cycle
-        // has a single vertex: its lowest one walks it, a warp a walk
+        // Nodes of several vertices choose single ones only, so every cycle
+        // has a single vertex: its lowest one walks it, a warp a walk, and
+        // writes down the cycle's lowest id and its number of nodes (par and
+        // skip, free by now).  No node is joined before all walks are done: a
+        // walk told the lowest single vertex by its node's size, and where a
+        // cycle was being joined could miss it, find the cycle a second time
+        // and write a second size.  (The barrier costs ~3 us a try.)
         for (int64_t i = gt; i - lane_id() < ns1; i += nt) {
             const int32_t mine = i < ns1 ? b.single[i] : 0;
-            int32_t first = mine;
+            int32_t first = mine, my_low = 0;
+            int my_len = 0;
             if (i < ns1 && !bitv(r.D, mine)) first = cyc_next(b, mine);
             for (unsigned g = __ballot_sync(kFull, first != mine && !(first < mine && __ldcg(b.size + first) == 1)); g;
                  g &= g - 1) {
@@ -395,9 +402,29 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
                         renew = 2 * len;
                     }
                 }
-                if (!found) continue;  // a lower single vertex, another cycle, too long, or no choice
-                int all = 0, fresh = 0;
-                int32_t w = v;
+                // (else: a lower single vertex, another cycle, too long, or no choice)
+                if (found && lane_id() == l) {
+                    my_low = low;
+                    my_len = len;
+                }
+            }
+            if (i < ns1) {
+                b.par[mine] = my_low;
+                b.skip[mine] = my_len;
+            }
+        }
+        if (!grid_sync(r.gsync, r.err)) return;
+        // the cycles found, which share no node, are joined, a warp a cycle
+        for (int64_t i = gt; i - lane_id() < ns1; i += nt) {
+            const int32_t mine = i < ns1 ? b.single[i] : 0;
+            const int my_len = i < ns1 ? __ldcg(b.skip + mine) : 0;
+            const int32_t my_low = my_len ? __ldcg(b.par + mine) : 0;
+            for (unsigned g = __ballot_sync(kFull, my_len > 0); g; g &= g - 1) {
+                const int l = __ffs(g) - 1;
+                const int len = __shfl_sync(kFull, my_len, l);
+                const int32_t low = __shfl_sync(kFull, my_low, l);
+                int32_t w = __shfl_sync(kFull, mine, l);
+                int all = 0, fresh = 0, dir = -1;
                 for (int k = 0; k < len;) {
                     const int c = min(cyc_run(r, b, w, dir), len - k);
                     const int32_t nw = c > 0 ? w + c * dir : cyc_next(b, w);  // (read before w's rep changes)

@@ -70,3 +70,24 @@ ASCENDING = {
 def test_minimum_that_leads_up(name, order):
     size, edges = ASCENDING[name]
     _check(_gadgets(1500, size, edges, dag=9000, seed=len(name), order=order))
+
+
+# a ring of several vertices with the lowest ids, from which a way of two (or
+# more) single vertices leads back to it: the cycle of nodes has its lowest id
+# in the ring and several single vertices that could each walk it.  Their ids
+# follow the way, run against it, or lie apart (rings between them)
+_RING = [(i, i + 1) for i in range(7)] + [(7, 0)]
+WAYS = {
+    "along": (10, _RING + [(7, 8), (8, 9), (9, 0)]),
+    "against": (10, _RING + [(7, 9), (9, 8), (8, 0)]),
+    "apart": (19, _RING + [(7, 8), (8, 18), (18, 0)] + [(i, i + 1) for i in range(9, 17)] + [(17, 9)]),
+}
+
+
+@pytest.mark.parametrize("name", list(WAYS))
+@pytest.mark.parametrize("order", ["up", "blocks"])
+def test_ways_back_to_the_lowest_ring(name, order):
+    """More single vertices (above 200,000) than threads, so that walks begin
+    at different times, over and over in one context."""
+    size, edges = WAYS[name]
+    _check(_gadgets(101_000, size, edges, dag=300_000, seed=len(name), order=order), runs=50)
