@@ -18,7 +18,8 @@
 //     in shared memory.  Larger ones are split again, kResIts times in all.
 //   Labelling (in a tile, and k_resolve for what is left): every vertex
 //     carries the lowest label among its ancestors, f, and among its
-//     descendants, b, inside its class (labels are the ids).  Where f = b =
+//     descendants, b, inside its class (labels are the ids, from the fourth
+//     round on mixed ones, see tile.cuh).  Where f = b =
 //     the label of p, p reaches the vertex and is reached from it: the vertex
 //     is in p's SCC, found without a separate backward search.  At least the
 //     SCC of each class's lowest label is.  The others go on, classed by
@@ -131,7 +132,8 @@ __device__ __forceinline__ int32_t res_near(const ResBufs &m, int d, int32_t v) 
 constexpr int kResU = 4;
 constexpr int kResLane = 64;
 template <int K>
-__device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int32_t (&v)[kResU]) {
+__device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int32_t (&v)[kResU],
+                                             const LabelMix<32> &mix) {
     using T = typename ResVal<K>::T;
     T *val = reinterpret_cast<T *>(m.val[d]);
     const int32_t *adj = m.adj[d];
@@ -148,7 +150,7 @@ __device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int3
     for (int u = 0; u < kResU; ++u) {
         nw[u] = own[u];
         if constexpr (K == R_MIN)
-            if (v[u] >= 0) nw[u] = min(own[u], __ldcg(val + own[u]));
+            if (v[u] >= 0) nw[u] = min(own[u], __ldcg(val + mix.holder(own[u])));
     }
     bool more = true;
     for (int step = 0; step < kResLane && more; step += 4) {
@@ -195,7 +197,8 @@ __device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int3
 // then jumps to its target's, which is read before the target's value (that
 // covers all between).  again: the link starts anew.
 template <int K>
-__device__ __forceinline__ bool res_pull_linked(const ResBufs &m, int d, int32_t v, uint32_t *link, bool again) {
+__device__ __forceinline__ bool res_pull_linked(const ResBufs &m, int d, int32_t v, uint32_t *link, bool again,
+                                                const LabelMix<32> &mix) {
     using T = typename ResVal<K>::T;
     T *val = reinterpret_cast<T *>(m.val[d]);
     const int32_t *adj = m.adj[d];
@@ -207,7 +210,7 @@ __device__ __forceinline__ bool res_pull_linked(const ResBufs &m, int d, int32_t
         const uint32_t far = __ldcg(link + v), to = __ldcg(link + far);
         own = __ldcg(val + v);
         nw = res_join<K>(own, __ldcg(val + far));
-        if constexpr (K == R_MIN) nw = min(nw, __ldcg(val + own));
+        if constexpr (K == R_MIN) nw = min(nw, __ldcg(val + mix.holder(own)));
         __stcg(link + v, again ? (uint32_t)res_near(m, d, v) : to);
     }
     const int32_t c = min(e, b + kResLane);
@@ -324,7 +327,7 @@ struct ResSmem {
 template <int K>
 __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &m, unsigned long long *chg,
                                            unsigned long long *qc, const unsigned long long *x_large, const int32_t *list, int64_t n, int dirs, int &s,
-                                           ResSmem &sm, bool seeded) {
+                                           ResSmem &sm, bool seeded, const LabelMix<32> &mix) {
     const int64_t gt = (int64_t)blockIdx.x * kBlock + threadIdx.x;
     const int64_t nt = (int64_t)gridDim.x * kBlock;
     bool dense = true;
@@ -363,7 +366,7 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
                     const int32_t v = i < n ? (list ? list[i] : (int32_t)i) : -1;
                     for (int d = 0; d < 2; ++d)
                         if ((dirs >> d) & 1)
-                            changed += res_pull_linked<K>(m, d, v, link[d], levels % kResAgain == kResAgain - 1);
+                            changed += res_pull_linked<K>(m, d, v, link[d], levels % kResAgain == kResAgain - 1, mix);
                 }
             const int64_t gw = gt >> 5, nw = nt >> 5;
             for (int64_t i0 = gw * (32 * kResU); i0 < n && !linked; i0 += nw * (32 * kResU)) {
@@ -375,7 +378,7 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
                 }
                 for (int d = 0; d < 2; ++d) {
                     if (!((dirs >> d) & 1)) continue;
-                    const unsigned ch = res_pull<K>(m, d, v);
+                    const unsigned ch = res_pull<K>(m, d, v, mix);
                     changed += __popc(ch);
                     if (!listing) continue;
                     unsigned g[kResU];
@@ -630,8 +633,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
             }
         }
         if (!grid_sync(r.gsync, r.err)) return;
-        const int ok = wide ? res_spread<R_OR64>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm, true)
-                            : res_spread<R_OR16>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm, true);
+        const int ok = wide ? res_spread<R_OR64>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm, true, LabelMix<32>(0))
+                            : res_spread<R_OR16>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 1 << d, s, sm, true, LabelMix<32>(0));
         if (ok == 0) return;
         if (ok == 2) {  // these masks say nothing; the labelling rounds take what no tile does
             if (gt == 0) x.ctl[K_RES_STOP] = 1ull;
@@ -845,21 +848,22 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
         int32_t *next = m.list[(kResIts + k) & 1];
         unsigned long long *n_next = left + k % 3;
         if (gt == 0) left[(k + 1) % 3] = 0ull;
+        const LabelMix<32> mix(k);
         for (int64_t i = gt; i < nl; i += nt) {
             const int32_t v = list[i];
-            m.val[0][v] = (uint32_t)v;
-            m.val[1][v] = (uint32_t)v;
+            m.val[0][v] = m.val[1][v] = mix.label((uint32_t)v);
             m.mn[v] = 0x7fffffff;
             m.size[v] = 0;
         }
         if (!grid_sync(r.gsync, r.err)) return;
-        if (res_spread<R_MIN>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 3, s, sm, false) != 1) return;
+        if (res_spread<R_MIN>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 3, s, sm, false, mix) != 1) return;
         for (int64_t i = gt; i < nl; i += nt) {
             const int32_t v = list[i];
             const uint32_t f = __ldcg(m.val[0] + v);
             if (f == __ldcg(m.val[1] + v)) {
-                atomicMin(m.mn + f, m.old[v]);
-                atomicAdd(m.size + f, 1);
+                const uint32_t p = mix.holder(f);
+                atomicMin(m.mn + p, m.old[v]);
+                atomicAdd(m.size + p, 1);
             }
         }
         if (!grid_sync(r.gsync, r.err)) return;
@@ -875,12 +879,12 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
                     m.cls[v] = mix32(f ^ mix32(b)) & 0x7fffffffu;
                 } else {
                     const int32_t ov = m.old[v];
-                    r.label[ov] = __ldcg(m.mn + f);
+                    r.label[ov] = __ldcg(m.mn + mix.holder(f));
                     r.cls[ov] = CLS_MICE;
                     clear_bit(r.A, ov);
                     m.cls[v] = kResDead;
                     ++done;
-                    if ((int32_t)f == v) {  // one histogram entry per SCC
+                    if ((int32_t)mix.holder(f) == v) {  // one histogram entry per SCC
                         const int32_t sz = __ldcg(m.size + v);
                         if (sz < kHistCap) {
                             atomicAdd((unsigned long long *)(r.hist + sz), 1ull);

@@ -31,10 +31,44 @@
 namespace ispan {
 
 constexpr int kTileAgain = 10;  // passes after which the links start anew: 2^10 hops
+constexpr int kRankRounds = 3;  // rounds with ranks as labels, here and in k_resolve
+
+// A permutation of the BITS-bit numbers and its inverse: odd factors (of the
+// golden ratio, as in multiplicative hashing) around an xor-shift by half the
+// width, which undoes itself.  Rounds below kRankRounds: the identity.
+template <int BITS>
+struct LabelMix {
+    static constexpr uint32_t kMask = BITS == 32 ? 0xffffffffu : (1u << (BITS & 31)) - 1u;
+    static constexpr int kShift = (BITS + 1) / 2;
+    uint32_t a, b, ia, ib;
+    bool on;
+    __device__ __forceinline__ explicit LabelMix(int round) : on(round >= kRankRounds) {
+        a = (0x9e3779b1u * (2u * (uint32_t)round + 1u)) | 1u;
+        b = ((0x9e3779b1u * (2u * (uint32_t)round + 2u)) >> 5) | 1u;
+        ia = a;
+        ib = b;
+        for (int k = 0; k < 4; ++k) {  // (Newton: 3 bits are right at first, twice as many each time)
+            ia *= 2u - a * ia;
+            ib *= 2u - b * ib;
+        }
+    }
+    __device__ __forceinline__ uint32_t label(uint32_t i) const {
+        if (!on) return i;
+        const uint32_t y = (i * a) & kMask;
+        return ((y ^ (y >> kShift)) * b) & kMask;
+    }
+    __device__ __forceinline__ uint32_t holder(uint32_t l) const {
+        if (!on) return l;
+        const uint32_t y = (l * ib) & kMask;
+        return ((y ^ (y >> kShift)) * ia) & kMask;
+    }
+};
 
 template <int V_, int E_, int THREADS>
 struct Tile {
     static constexpr int kV = V_, kE = E_, kThreads = THREADS, kPer = V_ / THREADS;
+    static constexpr int kBits = 31 - __builtin_clz(V_);  // of a local id
+    static_assert(V_ == 1 << kBits, "labels are mixed within the tile's ids");
     union {
         int32_t orig[V_];      // original ids; while solving:
         uint16_t link[2][V_];  // an ancestor, a descendant
@@ -113,12 +147,13 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
             if (tid == 0) atomicCAS(r.err, 0, kErrOverflow);
             break;
         }
+        const LabelMix<T::kBits> mix(round);
         // labels and links: the descendant nearest by id, and the reverse
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
             if (!((mine >> u) & 1u)) continue;
             const int i = u * T::kThreads + tid;
-            t.f[i] = t.b[i] = i;
+            t.f[i] = t.b[i] = (int32_t)mix.label(i);
             t.link[0][i] = (uint16_t)i;
         }
         __syncthreads();
@@ -144,8 +179,8 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
                 volatile uint16_t *anc = t.link[0], *des = t.link[1];
                 const int la = anc[i], ld = des[i];
                 const uint16_t la2 = anc[la], ld2 = des[ld];
-                const int32_t fv = min(min(f0, f[f0]), f[la]);
-                int32_t bv = min(min(b0, b[b0]), b[ld]);
+                const int32_t fv = min(min(f0, f[mix.holder(f0)]), f[la]);
+                int32_t bv = min(min(b0, b[mix.holder(b0)]), b[ld]);
                 const int o = t.off[i], z = o + t.len[i];
                 for (int k = o; k < z; ++k) {
                     const int w = t.adj[k];
@@ -162,9 +197,9 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
                 }
             }
         }
-        // solved: f = b = p.  A solved p gathers its SCC's lowest
-        // original id in f[p] and its size in b[p] (its members keep p in
-        // their own f)
+        // solved: f = b = p's label.  A solved p gathers its SCC's lowest
+        // original id in f[p] and its size in b[p] (its members keep
+        // p's label in their own f)
         unsigned sol = 0;
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
@@ -174,7 +209,8 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
         unsigned roots = 0;
 #pragma unroll
         for (int u = 0; u < kPer; ++u)
-            if (((sol >> u) & 1u) && t.f[u * T::kThreads + tid] == u * T::kThreads + tid) roots |= 1u << u;
+            if (((sol >> u) & 1u) && (int)mix.holder(t.f[u * T::kThreads + tid]) == u * T::kThreads + tid)
+                roots |= 1u << u;
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
@@ -190,7 +226,7 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
         for (int u = 0; u < kPer; ++u) {
             const int i = u * T::kThreads + tid;
             if (((sol & ~roots) >> u) & 1u) {
-                const int p = t.f[i];
+                const int p = (int)mix.holder(t.f[i]);
                 atomicMin(&t.f[p], orig[u]);
                 atomicAdd(&t.b[p], 1);
             }
@@ -201,7 +237,7 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
             const int i = u * T::kThreads + tid;
             if (!((sol >> u) & 1u)) continue;
             const bool root = (roots >> u) & 1u;
-            const int32_t lab = root ? t.f[i] : t.f[t.f[i]], ov = orig[u];
+            const int32_t lab = root ? t.f[i] : t.f[mix.holder(t.f[i])], ov = orig[u];
             r.label[ov] = lab;
             r.cls[ov] = CLS_MICE;
             clear_bit(r.A, ov);
