@@ -38,7 +38,17 @@ constexpr int kSmallWords = kSmallV / 32;
 constexpr int kSmallOwn = kSmallWords / kSmallCtas;  // words a CTA owns, at most
 constexpr int kSmallLane = 16;            // entries of a list a lane reads alone
 constexpr int kSmallHub = 4096;           // a longer list is pushed by the whole CTA
-constexpr int kSmallSteps = 12;           // steps of a push inside a CTA before the cluster meets
+// Steps of a push inside a CTA before the cluster meets: more while the whole
+// cluster's frontier is a few vertices (a ring of 60,000: 95 ms by 12 steps, 74
+// by 128, 72 by 1,024); none once the CTA's own frontier is wide: apart, each CTA
+// would then walk most of the graph by itself.  Uniform random graphs of 30,000
+// to 65,000 vertices and 0.5 to 4 M edges: 0.41-1.02 ms without that limit,
+// 0.12-0.23 with it (0.21-0.41 by the stage kernels).  64 to 1,024 vertices are
+// alike there; on a grid of 250 x 250 256 took 2.53 ms and 1,024 1.35, on six
+// planted-cycle graphs of 2,000 to 12,000 vertices 64 took 0.81 and 1,024 0.67.
+constexpr int kSmallSteps = 12;
+constexpr int kSmallFew = 32, kSmallFewSteps = 128;
+constexpr int kSmallWide = 1024;
 constexpr int kSmallQ = 4096;             // vertices a CTA goes on with; more are left to their owners
 
 struct SmallSmem {
@@ -248,7 +258,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(Run<OffT> r, Ext<Off
         }
     }
     // both searches, level by level.  A small frontier pushes along its lists
-    // and goes on from what it marked for kSmallSteps steps, each CTA by
+    // and goes on from what it marked for some steps (kSmallSteps), each CTA by
     // itself, before the cluster meets; a wide one is pulled: each unreached
     // vertex looks for a reached one
     int64_t front[2] = {n_piv, n_piv};
@@ -322,7 +332,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(Run<OffT> r, Ext<Off
                 m = __shfl_sync(kFull, m, 0);
                 if ((m >> lane) & 1u) small_list(s, r, d, (w0 + k) * 32 + lane);
             }
-            for (int step = 0; step < kSmallSteps; ++step) {
+            const int steps = front[0] + front[1] <= kSmallFew ? kSmallFewSteps : kSmallSteps;
+            for (int step = 0; step < steps; ++step) {
                 const int nq = min(s.nq, kSmallQ);
                 for (int i = tid; i < nq; i += kSmallThreads) {
                     const uint32_t ent = s.q[i];
@@ -337,6 +348,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(Run<OffT> r, Ext<Off
                 __syncthreads();
                 if (tid < 3) s.n[tid] = 0;
                 __syncthreads();
+                if (s.nq > kSmallWide) break;
             }
             __syncthreads();
             nq_left = min(s.nq, kSmallQ);
