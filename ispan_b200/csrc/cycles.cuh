@@ -681,7 +681,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_super(Run<OffT> r, Ext<OffT> x, C
     const int lane = lane_id();
     const int32_t *L = x.large[0];
     unsigned long long *qc = x.ctl + K_SUP_Q;  // 3 rotating counters
-    // spans of the descending edges: +1 at the lower node, -1 behind the upper
+    // spans of the descending edges: +1 at the lower node, -1 behind the upper.
+    // A vertex has one for all of its edges, to the farthest of them, which
+    // covers the others: counts stay below the number of vertices (int32),
+    // however many edges there are
     const bool flip = __ldcg(x.ctl + K_CYC_ON) == 2ull;
     int32_t *diff = r.cnt_in;
     const int64_t per = ((r.W + gridDim.x - 1) / gridDim.x) * 32;  // ids per CTA, whole words
@@ -690,6 +693,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_super(Run<OffT> r, Ext<OffT> x, C
     if (!grid_sync(r.gsync, r.err)) return;
     for (int64_t i = gt; i < n; i += nt) {
         const int32_t v = L[i], rv = __ldcg(b.rep + v);
+        int32_t far = rv;
         for (int64_t e = ld_off(r.fw_beg, v), e1 = ld_off(r.fw_beg, v + 1); e < e1; e += 4) {
             int32_t w[4], rw[4];
 #pragma unroll
@@ -697,11 +701,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_super(Run<OffT> r, Ext<OffT> x, C
 #pragma unroll
             for (int q = 0; q < 4; ++q) rw[q] = w[q] != v && bitc(r.A, w[q]) ? __ldcg(b.rep + w[q]) : rv;
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (flip ? rw[q] > rv : rw[q] < rv) {
-                    atomicAdd(diff + min(rv, rw[q]), 1);
-                    atomicAdd(diff + max(rv, rw[q]) + 1, -1);
-                }
+            for (int q = 0; q < 4; ++q) far = flip ? max(far, rw[q]) : min(far, rw[q]);
+        }
+        if (far != rv) {
+            atomicAdd(diff + min(rv, far), 1);
+            atomicAdd(diff + max(rv, far) + 1, -1);
         }
     }
     if (!grid_sync(r.gsync, r.err)) return;

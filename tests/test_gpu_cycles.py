@@ -91,3 +91,19 @@ def test_ways_back_to_the_lowest_ring(name, order):
     at different times, over and over in one context."""
     size, edges = WAYS[name]
     _check(_gadgets(101_000, size, edges, dag=300_000, seed=len(name), order=order), runs=50)
+
+
+@pytest.mark.parametrize("order", ["up", "down", "blocks"])
+@pytest.mark.parametrize("copies", [1, 40])
+def test_spans_of_many_edges(order, copies):
+    """Vertices with many edges against the order, near and far, each `copies`
+    times: a vertex has one span, to the farthest."""
+    rng = np.random.default_rng(copies)
+    csr = _gadgets(900, 40, [(i, (i + 1) % 40) for i in range(40)], dag=4000, seed=5, order=order)
+    src = np.repeat(np.arange(csr.V), np.diff(csr.fw_beg))
+    n = 900 * 40
+    # back edges over spans of up to 60 rings, from few vertices
+    v = rng.integers(0, n, 150).repeat(12)
+    w = np.maximum(0, v - rng.integers(0, 2400, len(v)))
+    csr = _csr(csr.V, np.concatenate([src, np.tile(v, copies)]), np.concatenate([csr.fw_adj, np.tile(w, copies)]))
+    _check(csr)
