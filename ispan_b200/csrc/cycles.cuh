@@ -232,11 +232,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
     if (n < kCycMin) return;
     const int32_t *wl = r.wl[0];
     // the sample: every CTA takes the same one, so all agree without a barrier
-    __shared__ int s_near, s_down;
-    if (threadIdx.x == 0) s_near = s_down = 0;
+    __shared__ int s_near;
+    if (threadIdx.x == 0) s_near = 0;
     __syncthreads();
     const int ns = (int)min(n, (int64_t)kCycSample);
-    int near = 0, down = 0, up = 0;
+    int near = 0;
     for (int k = threadIdx.x; k < ns; k += kBlock) {
         const int32_t v = wl[(int64_t)k * n / ns];
         bool has = false;
@@ -244,21 +244,14 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
             const int32_t u = ld_adj(r.bw_adj, e);
             if (u == v || !bitc(r.A, u)) continue;
             has |= abs((long long)u - v) <= kCycNear;
-            down += u > v;
-            up += u < v;
         }
         near += has;
     }
     near = __reduce_add_sync(kFull, near);
-    down = __reduce_add_sync(kFull, down);
-    up = __reduce_add_sync(kFull, up);
-    if (lane_id() == 0) {
-        atomicAdd(&s_near, near);
-        atomicAdd(&s_down, down - up);
-    }
+    if (lane_id() == 0) atomicAdd(&s_near, near);
     __syncthreads();
     if (4 * s_near < ns) return;
-    if (gt == 0) x.ctl[K_CYC_ON] = s_down > 0 ? 2ull : 1ull;  // 2: most edges lead down, k_super looks from below
+    if (gt == 0) x.ctl[K_CYC_ON] = 1ull;
     // pointers, by words of the active map (P, D: pointers to the id before,
     // to the one after)
     for (int64_t w = gt >> 5; w < r.W; w += nt >> 5) {
@@ -685,7 +678,28 @@ __global__ void __launch_bounds__(kBlock, 2) k_super(Run<OffT> r, Ext<OffT> x, C
     // A vertex has one for all of its edges, to the farthest of them, which
     // covers the others: counts stay below the number of vertices (int32),
     // however many edges there are
-    const bool flip = __ldcg(x.ctl + K_CYC_ON) == 2ull;
+    // Which way descends: the way that fewer edges between nodes go, of a
+    // sample of the list that every CTA takes alike.  (Edges inside a node say
+    // nothing: a line of 40,000 SCCs, half of them rings whose edges lead up, with
+    // ids down the line: 432 ms when judged by all edges, 0.5 a line of rings.)
+    __shared__ int s_down;
+    if (threadIdx.x == 0) s_down = 0;
+    __syncthreads();
+    const int ns = (int)min(n, (int64_t)kCycSample);
+    int down = 0;
+    for (int k = threadIdx.x; k < ns; k += kBlock) {
+        const int32_t v = L[(int64_t)k * n / ns], rv = __ldcg(b.rep + v);
+        for (int64_t e = ld_off(r.fw_beg, v), e1 = min(ld_off(r.fw_beg, v + 1), e + 16); e < e1; ++e) {
+            const int32_t w = ld_adj(r.fw_adj, e);
+            if (w == v || !bitc(r.A, w)) continue;
+            const int32_t rw = __ldcg(b.rep + w);
+            down += rw < rv ? 1 : rw > rv ? -1 : 0;
+        }
+    }
+    down = __reduce_add_sync(kFull, down);
+    if (lane == 0) atomicAdd(&s_down, down);
+    __syncthreads();
+    const bool flip = s_down > 0;
     int32_t *diff = r.cnt_in;
     const int64_t per = ((r.W + gridDim.x - 1) / gridDim.x) * 32;  // ids per CTA, whole words
     const int64_t c0 = min(r.V + 1, (int64_t)blockIdx.x * per), c1 = min(r.V + 1, c0 + per);

@@ -31,7 +31,7 @@ enum Ctl64 {
     K_TICKET1,                     // with k_local_scc (see set_gate)
     K_MID, K_MID_BACK,             // WCCs with a tile of their own, their vertices
     K_SMALL_DONE,                  // 1: k_small wrote all labels; the finalisation returns at once
-    K_CYC_ON, K_CYC_N, K_CYC_MEM, K_CYC_LEFT,  // cycles.cuh: cycles were looked for (2: most edges lead down),
+    K_CYC_ON, K_CYC_N, K_CYC_MEM, K_CYC_LEFT,  // cycles.cuh: cycles were looked for,
                                    // vertices on those found, places taken, vertices on none,
     K_SUP_Q, K_SUP_LEFT = K_SUP_Q + 3,  // vertices to peel (3 slots), vertices left
     kNumCtl = 72
