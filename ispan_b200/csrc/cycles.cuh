@@ -45,6 +45,7 @@ constexpr int64_t kCycMin = 1 << 15;  // fewer residual vertices: most WCCs fit 
 constexpr int kCycSample = 2048;    // residual vertices sampled
 constexpr int kCycNear = 1024;      // an in-neighbour this near counts; a quarter of the sample must have one
 constexpr int kCycMax = 1 << 12;    // longest walk, in runs of consecutive ids (later: in nodes)
+constexpr int kCycSteps = 64;       // steps (32 consecutive ids, or a node) of a walk over nodes while ids are its priorities
 constexpr int kCycTries = 2;        // times the nodes choose again, while single vertices are joined
 constexpr int kSuperTail = 1024;    // a round of the peel of at most this many vertices: one CTA alone
 constexpr int kSuperTailRounds = 256;
@@ -280,15 +281,22 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
         const int32_t v = wl[i];
         int32_t u = __ldcg(b.par + v), h = v;
         if (u <= v) continue;
-        int hops = 0, len = 0;
-        for (; hops < kCycMax && u > v; ++hops) {
+        int hops = 0, len = 0, renew = 1;
+        // (a mark renewed at powers of two: met again, the walk is in a cycle of
+        // higher ids, without v)
+        for (int32_t mark = u; hops < kCycMax && u > v; ++hops) {
             h = __ldcg(b.skip + u);
             len += abs(u - h) + 1;
             if (h <= v) break;  // v ends descending runs, its own pointer leads up
             u = __ldcg(b.par + h);
+            if (u == mark) break;
+            if (hops == renew) {
+                mark = u;
+                renew *= 2;
+            }
         }
         if (u == v) ++len;
-        else if (h != v) continue;  // met a lower id, or too long
+        else if (h != v) continue;  // met a lower id or another cycle, or too long
         u = __ldcg(b.par + v);
         for (int k = 0; k <= hops; ++k) {
             h = u == v ? v : __ldcg(b.skip + u);
@@ -329,6 +337,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
     int64_t joined = 0;
     for (int64_t i = gt; i < n; i += nt) b.key[wl[i]] = ~0ull;  // the first walks' marks
     if (!grid_sync(r.gsync, r.err)) return;
+    bool hashed = false;  // the walks' priorities: ids, or a hash of them
     for (int t = 0; t < kCycTries && joined < ns1; ++t) {
         if (t) {
             for (int64_t i = gt; i < ns1; i += nt) {
@@ -347,36 +356,54 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
         }
         if (!grid_sync(r.gsync, r.err)) return;
         // Nodes of several vertices choose single ones only, so every cycle
-        // has a single vertex: its lowest one walks it, a warp a walk, and
-        // writes down the cycle's lowest id and its number of nodes (par and
-        // skip, free by now).  No node is joined before all walks are done: a
-        // walk told the lowest single vertex by its node's size, and where a
-        // cycle was being joined could miss it, find the cycle a second time
-        // and write a second size.  (The barrier costs ~3 us a try.)
+        // has a single vertex: the one of the lowest priority walks it, a warp
+        // a walk, and writes down the cycle's lowest id and its number of nodes
+        // (par and skip, free by now).  A walk ends at a single vertex of lower
+        // priority.  The ids are the priorities (most walks then end at once
+        // where ids follow the rings; hashes from the start cost 97 graphs in
+        // one call 0.4 ms of 4), for kCycSteps steps at most: up a way whose
+        // ids ascend every walk would go on and on.  If any did, the next try
+        // takes a hash of the ids: on a way of any length a walk goes a few
+        // steps, the logarithm of it.  (Ids and kCycMax steps: a line of 200,000
+        // rings and single vertices whose ids ascend 639 ms, of 20,000 301; so
+        // 19 and 12.)
+        // No node is joined before all walks are done: a walk told that single
+        // vertex by its node's size, and where a cycle was being joined could
+        // miss it, find the cycle a second time and write a second size.  (The
+        // barrier costs ~3 us a try.)
+        const auto prio = [hashed](int32_t a) { return hashed ? prio_of((uint32_t)a) : (uint32_t)a; };
         for (int64_t i = gt; i - lane_id() < ns1; i += nt) {
             const int32_t mine = i < ns1 ? b.single[i] : 0;
             int32_t first = mine, my_low = 0;
             int my_len = 0;
             if (i < ns1 && !bitv(r.D, mine)) first = cyc_next(b, mine);
-            for (unsigned g = __ballot_sync(kFull, first != mine && !(first < mine && __ldcg(b.size + first) == 1)); g;
-                 g &= g - 1) {
+            for (unsigned g = __ballot_sync(kFull, first != mine && !(__ldcg(b.size + first) == 1 && prio(first) < prio(mine)));
+                 g; g &= g - 1) {
                 const int l = __ffs(g) - 1;
                 const int32_t v = __shfl_sync(kFull, mine, l);
+                const uint32_t pv = prio(v);
                 int32_t u = __shfl_sync(kFull, first, l), low = v, mark = u;
-                int len = 1, dir = -1, renew = 2;
+                int len = 1, dir = -1, renew = 2, steps = 0;
                 bool found = false;
                 // (a mark renewed at powers of two: met again, the walk is in a cycle without v)
-                while (len < kCycMax && !(u < v && __ldcg(b.size + u) == 1)) {
+                while (len < kCycMax && !(__ldcg(b.size + u) == 1 && prio(u) < pv)) {
+                    if (!hashed && ++steps > kCycSteps) {
+                        x.ctl[K_CYC_CUT] = 1ull;
+                        break;
+                    }
                     low = min(low, u);
                     const int c = cyc_run(r, b, u, dir);
                     if (c > 0) {
                         const int64_t jv = ((int64_t)v - u) * dir, jm = ((int64_t)mark - u) * dir;
-                        if (jv >= 1 && jv <= c) {
+                        const unsigned lower =
+                            __ballot_sync(kFull, lane_id() > 0 && lane_id() <= c && prio(u + lane_id() * dir) < pv);
+                        const int jl = lower ? __ffs(lower) - 1 : c + 1;
+                        if (jv >= 1 && jv <= c && jv < jl) {
                             len += (int)jv;
                             found = true;
                             break;
                         }
-                        if (jm >= 1 && jm <= c) break;
+                        if (jl <= c || (jm >= 1 && jm <= c)) break;
                         u += c * dir;
                         len += c;
                     } else {
@@ -395,7 +422,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
                         renew = 2 * len;
                     }
                 }
-                // (else: a lower single vertex, another cycle, too long, or no choice)
+                // (else: a single vertex of lower priority, another cycle, too long, or no choice)
                 if (found && lane_id() == l) {
                     my_low = low;
                     my_len = len;
@@ -443,7 +470,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
         }
         if (!grid_sync(r.gsync, r.err)) return;
         const int64_t now = (int64_t)__ldcg(x.ctl + K_CYC_N);
-        if (now == joined) break;
+        hashed = __ldcg(x.ctl + K_CYC_CUT) != 0;
+        if (now == joined && !hashed) break;
         joined = now;
     }
     if (joined == 0) return;

@@ -75,6 +75,7 @@ struct ResBufs {
     int32_t *pos;           // [n] place of a vertex in order (overlays val[0])
 };
 
+// lowbias32, the 32-bit integer hash of C. Wellons' hash prospector
 __device__ __forceinline__ uint32_t mix32(uint32_t h) {
     h ^= h >> 16;
     h *= 0x7feb352du;

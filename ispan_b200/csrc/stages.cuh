@@ -34,6 +34,7 @@ enum Ctl64 {
     K_CYC_ON, K_CYC_N, K_CYC_MEM, K_CYC_LEFT,  // cycles.cuh: cycles were looked for,
                                    // vertices on those found, places taken, vertices on none,
     K_SUP_Q, K_SUP_LEFT = K_SUP_Q + 3,  // vertices to peel (3 slots), vertices left
+    K_CYC_CUT,                     // 1: a walk over nodes was cut short
     kNumCtl = 72
 };
 
@@ -1119,7 +1120,8 @@ __global__ void __launch_bounds__(TileSmem::kThreads) k_local_scc(Run<OffT> r, E
 // ring-shaped SCCs cost no grid barrier per hop.
 __device__ __forceinline__ uint32_t prio_of(uint32_t v) {
     // bijection on [0, 2^31): xor-shifts and odd multipliers mod 2^31 are
-    // invertible there
+    // invertible there (the steps and factors of lowbias32, C. Wellons' hash
+    // prospector, mod 2^31)
     v &= 0x7fffffffu;
     v ^= v >> 16;
     v = (v * 0x7feb352du) & 0x7fffffffu;

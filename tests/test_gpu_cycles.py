@@ -126,3 +126,37 @@ def test_line_of_rings_either_way(ring, order):
         t = time.perf_counter()
         ctx.run_csr(csr)
         assert time.perf_counter() - t < 0.05
+
+
+# walks that lead into cycles they are not on, or up a long way: gadgets of a ring
+# and a vertex below it, alone and in a line whose ids ascend
+@pytest.mark.parametrize("line", [False, True])
+@pytest.mark.parametrize("step", [1, 7])
+def test_walks_beside_rings(line, step):
+    import time
+    from ispan_b200 import Context
+    L, k = 20, 50_000
+    edges = [(1 + i, 1 + (i + step) % L) for i in range(L)] + [(5, 0)] + ([] if line else [(0, 7)])
+    size = L + 1
+    if line:  # the vertex below leads to the ring of the copy before
+        e = np.array(edges)
+        base = np.arange(k) * size
+        S = [(base[:, None] + e[None, :, 0]).ravel(), base[1:], [0], [k * size]]
+        D = [(base[:, None] + e[None, :, 1]).ravel(), base[:-1] + 3, [3], [k * size]]
+        h = 1200
+        n = k * size
+        S += [np.full(h, n), n + 1 + np.arange(h)]
+        D += [n + 1 + np.arange(h), np.full(h, n)]
+        csr = _csr(n + h + 1, np.concatenate(S), np.concatenate(D))
+    else:
+        e = np.array(edges)
+        base = np.arange(k) * size
+        n, h = k * size, 1200
+        csr = _csr(n + h + 1, np.concatenate([(base[:, None] + e[None, :, 0]).ravel(), np.full(h, n), n + 1 + np.arange(h)]),
+                   np.concatenate([(base[:, None] + e[None, :, 1]).ravel(), n + 1 + np.arange(h), np.full(h, n)]))
+    _check(csr)
+    with Context(csr.V, csr.E) as ctx:
+        ctx.run_csr(csr)
+        t = time.perf_counter()
+        ctx.run_csr(csr)
+        assert time.perf_counter() - t < 0.1  # (the line with ids as priorities: 0.3 s and more)
