@@ -300,9 +300,10 @@ __device__ __forceinline__ void res_push(const ResBufs &m, bool have, uint32_t e
 // the fixpoint in the directions of `dirs` (bit 0 forward, bit 1 backward).
 // s: the rotating counter slot; seeded: the vertices that hold a value are
 // listed already (q[0], their number in the slot).  Returns 1; 0 if a grid barrier failed; 2 if
-// it gave up, which only masks do, after about kResBudget levels: on long
-// paths without shortcuts they come one edge far per level, where labels jump
-// (after kResHops levels the labels take dense passes again).
+// it gave up, which only masks do, after about kResBudget levels or kResPasses
+// dense passes: on long paths without shortcuts they come one edge far per
+// level, where labels jump (after kResHops levels the labels take dense passes
+// again).
 //   dense passes while many vertices change;
 //   levels of listed vertices over the whole grid, then,
 //   while a level has at most kResTail of them, levels in CTA 0 alone,
@@ -311,6 +312,9 @@ __device__ __forceinline__ void res_push(const ResBufs &m, bool have, uint32_t e
 constexpr int kResTail = 1024;
 constexpr int kResTailLevels = 256;  // levels in CTA 0 before the grid meets again
 constexpr int kResBudget = 1024;
+constexpr int kResPasses = 160;  // (web graphs: up to 40, rings of 300 with shuffled ids 140; grids both ways, one
+                                 // SCC: 450, in each of up to 7 rounds.  400 x 400: 18-30 ms a call, so 4-5;
+                                 // 1,000 x 1,000 with shuffled ids 27-29, so 18)
 constexpr int kResHops = 64;
 // Few vertices take dense passes to the end, over links too (see Tile): a pass
 // costs what a level does, ~9 us, and the links end rings of a thousand hops
@@ -333,7 +337,7 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
     const int64_t nt = (int64_t)gridDim.x * kBlock;
     bool dense = true;
     int64_t prev = n * 2, nq = 0;
-    int cur = 0, levels = 0, hops = 0;
+    int cur = 0, levels = 0, hops = 0, passes = 0;
     // few vertices: links, and dense passes to the end
     const bool linked = n <= kResLinkN;
     uint32_t *link[2] = {nullptr, nullptr};
@@ -357,7 +361,7 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
     for (int64_t guard = 0; guard <= 128 * (r.V + 2); ++guard) {  // every pass lowers a value or sets a bit
         const int s1 = s == 2 ? 0 : s + 1;
         if (blockIdx.x == 0 && threadIdx.x == 0) { chg[s1] = 0ull; qc[s1] = 0ull; }
-        if (K != R_MIN && levels > kResBudget) return 2;
+        if (K != R_MIN && (levels > kResBudget || passes > kResPasses)) return 2;
         if (dense) {
             // few changes in the last pass: the vertices that change now are listed
             const bool listing = prev <= n / kResSparse && !linked;
@@ -410,6 +414,7 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
             if (prev == 0) return 1;
             if (listing && nq <= m.cap_q) { dense = false; cur = hops = 0; }
             ++levels;
+            ++passes;
             continue;
         }
         const uint32_t *qi = m.q[cur];
@@ -587,7 +592,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
     unsigned long long *work = x.ctl + K_RES_WORK + kResWork * it;
     int32_t *uf = reinterpret_cast<int32_t *>(m.cls);
     int32_t *cnt = m.mn, *base = m.size;
-    if (it && (nl < n / kResFew || __ldcg(x.ctl + K_RES_STOP))) {  // the labelling rounds take what is left
+    // the labelling rounds take what is left if it is little, or if the last time
+    // ended next to nothing: one SCC, on which masks are lost
+    const int64_t before = it > 1 ? (int64_t)__ldcg(x.ctl + K_RES_LEFT + it - 2) : n;
+    if (it && (nl < n / kResFew || 10 * nl > 9 * before || __ldcg(x.ctl + K_RES_STOP))) {
         for (int64_t i = gt; i < nl; i += nt) m.list[it & 1][i] = list[i];
         if (gt == 0) x.ctl[K_RES_LEFT + it] = (unsigned long long)nl;
         return;

@@ -77,3 +77,31 @@ def test_low_ids_at_both_ends(k, copies):
         ctx.run_csr(csr)
         if copies == 1 and k <= 2000:  # one tile: 25 rounds of at most 2 ms
             assert time.perf_counter() - t < 0.1
+
+
+# one SCC outside the pivot's whose diameter is hundreds of edges, below and
+# above the size up to which values spread over links: masks of pivots say
+# nothing on it, and are given up within the first round
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [400, 600])
+@pytest.mark.parametrize("ids", ["rows", "mixed"])
+def test_masks_given_up(k, ids):
+    import oracle
+    from ispan_b200 import Context
+    from test_gpu_resolve import _csr
+    i = np.arange(k * k)
+    r, d = i[i % k < k - 1], i[:-k]
+    n, h = k * k, 1200
+    S, D = np.concatenate([r, d, r + 1, d + k]), np.concatenate([r + 1, d + k, r, d])
+    if ids == "mixed":
+        p = np.random.default_rng(k).permutation(n)
+        S, D = p[S], p[D]
+    csr = _csr(5 * (n + h + 1), np.concatenate([S, np.full(h, n), n + 1 + np.arange(h)]),
+               np.concatenate([D, n + 1 + np.arange(h), np.full(h, n)]))
+    exact = oracle.tarjan(csr)
+    with Context(csr.V, csr.E) as ctx:
+        for graph in (True, False):
+            labels, st = ctx.run_csr(csr, histogram=True, use_graph=graph)
+            assert np.array_equal(labels, exact)
+            assert st["histogram"] == oracle.histogram(exact)
+            assert st["color_rounds"] <= 2  # (4 to 8 before)
