@@ -393,6 +393,7 @@ static void fill_run(ispan_ctx *c, Run<OffT> &r, Ext<OffT> &x, int64_t V, int64_
     x.large[1] = c->large[1];
     x.cq[0] = c->qv[0];  // the frontier queues are free once the giant is done
     x.cq[1] = c->qv[1];
+    x.nsm = c->nsm;
     x.cand = c->small;   // free until the WCC stage lists its small components
 }
 

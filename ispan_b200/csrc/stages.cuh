@@ -59,6 +59,7 @@ struct Ext {
     int32_t *large[2];            // [V] vertices of large WCCs (double buffered)
     int32_t *cq[2];               // [V] peel cascade queues
     int32_t *cand;                // [V] trim-2/3 candidates left by the first peel (count K_CAND)
+    int nsm;                      // the device's SMs: k_local_scc has a CTA on each
     // captured runs: gates of the conditional parts of the graph (0: none)
     cudaGraphConditionalHandle gate_left, gate_large;
 };
@@ -630,9 +631,9 @@ __global__ void __launch_bounds__(kBlock) k_trim3(Run<OffT> r, Ext<OffT> x, cons
 }
 
 // members per tile: short enough that a small residual spreads over the SMs
-__device__ __forceinline__ int wcc_tile(int64_t n) {
+__device__ __forceinline__ int wcc_tile(int64_t n, int nsm) {
     int t = kTileT;
-    while (t > 256 && n <= 148ll * (t / 2)) t >>= 1;
+    while (t > 256 && n <= (int64_t)nsm * (t / 2)) t >>= 1;
     return t;
 }
 
@@ -679,7 +680,7 @@ __global__ void __launch_bounds__(kBlock) k_wcc_init(Run<OffT> r, Ext<OffT> x, i
         r.aux2[v] = -1;    // member base of a small WCC
         r.cnt_out[v] = 0;  // fill cursor
     }
-    const int64_t tiles = n / wcc_tile(n) + 1;  // first WCC of each tile of the member list
+    const int64_t tiles = n / wcc_tile(n, x.nsm) + 1;  // first WCC of each tile of the member list
     for (int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x; i < tiles; i += (int64_t)gridDim.x * kBlock)
         x.large[1][i] = 0x7fffffff;
     // a batch's per-graph giant roots are marked in D (free after the peels)
@@ -866,7 +867,7 @@ __global__ void __launch_bounds__(kBlock) k_wcc_alloc(Run<OffT> r, Ext<OffT> x) 
     pdl_trigger();
     if (__ldcg(x.ctl + K_TINY)) return;  // the residual was solved in one CTA
     const int64_t n = (int64_t)__ldcg(x.ctl + K_ROOTS), nv = (int64_t)__ldcg(x.ctl + K_WL0);
-    const int per = wcc_tile(nv);
+    const int per = wcc_tile(nv, x.nsm);
     for (int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x; i - threadIdx.x < n;
          i += (int64_t)gridDim.x * kBlock) {
         const int32_t v = i < n ? x.roots[i] : 0, c = i < n ? r.aux[v] : 0;
@@ -943,7 +944,7 @@ __global__ void __launch_bounds__(TileSmem::kThreads) k_local_scc(Run<OffT> r, E
     T &t = *reinterpret_cast<T *>(tile_raw);
     const int tid = threadIdx.x, lane = lane_id();
     const int64_t total = (int64_t)__ldcg(x.ctl + K_ALLOC), mids = (int64_t)__ldcg(x.ctl + K_MID);
-    const int per = wcc_tile((int64_t)__ldcg(x.ctl + K_WL0));
+    const int per = wcc_tile((int64_t)__ldcg(x.ctl + K_WL0), x.nsm);
     const int64_t tiles = (total + per - 1) / per;
     const int32_t *first = x.large[1];
     int64_t done = 0, sccs = 0;
