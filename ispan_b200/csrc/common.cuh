@@ -123,7 +123,8 @@ constexpr int kErrOverflow = ISPAN_ERR_INTERNAL;
 // adjacency position and queue slot is range-checked against the run's sizes;
 // the first violation is recorded (site, index) and the access is skipped, so
 // a bad index reports instead of faulting.  The normal build compiles the
-// checks away.
+// checks away.  The sizes are one set per process: a checked build runs one
+// context at a time (a server's lanes would check against one another's).
 #ifdef ISPAN_CHECKED
 __device__ long long g_vcap, g_ecap, g_qcap;  // V, E, chunk-table entries
 __device__ long long g_chk[2];                // first violation: site, index

@@ -192,12 +192,18 @@ __global__ void __launch_bounds__(kBlock) k_cmp_fill(Run<OffT> r, Ext<OffT> x, C
         int64_t p = b.fbeg[i];
         for (int64_t e = ld_off(r.fw_beg, v), e1 = ld_off(r.fw_beg, v + 1); e < e1; ++e) {
             const int32_t w = ld_adj(r.fw_adj, e);
-            if (w != v && bitc(r.A, w)) b.fadj[p++] = __ldcg(b.newid + w);
+            if (w != v && bitc(r.A, w)) {
+                if (ICHK(p < b.cap_e, 43, p)) b.fadj[p] = __ldcg(b.newid + w);
+                ++p;
+            }
         }
         p = b.bbeg[i];
         for (int64_t e = ld_off(r.bw_beg, v), e1 = ld_off(r.bw_beg, v + 1); e < e1; ++e) {
             const int32_t w = ld_adj(r.bw_adj, e);
-            if (w != v && bitc(r.A, w)) b.badj[p++] = __ldcg(b.newid + w);
+            if (w != v && bitc(r.A, w)) {
+                if (ICHK(p < b.cap_e, 43, p)) b.badj[p] = __ldcg(b.newid + w);
+                ++p;
+            }
         }
     }
 }

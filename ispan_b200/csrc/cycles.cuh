@@ -86,7 +86,9 @@ __device__ __forceinline__ int32_t nearest_in(const Run<OffT> &r, int32_t v) {
 }
 
 __device__ __forceinline__ int32_t cyc_node(const CycBufs &b, int32_t v) {  // v's node (joined ones follow one another)
+    if (!VOK(v, 34)) return 0;
     int32_t a = __ldcg(b.rep + v);
+    if (!VOK(a, 35)) return 0;
     for (int32_t c; (c = __ldcg(b.rep + a)) != a;) a = c;
     return a;
 }
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
         // higher ids, without v)
         for (int32_t mark = u; hops < kCycMax && u > v; ++hops) {
             h = __ldcg(b.skip + u);
+            if (!VOK(h, 39)) break;
             len += abs(u - h) + 1;
             if (h <= v) break;  // v ends descending runs, its own pointer leads up
             u = __ldcg(b.par + h);
@@ -300,6 +303,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
         u = __ldcg(b.par + v);
         for (int k = 0; k <= hops; ++k) {
             h = u == v ? v : __ldcg(b.skip + u);
+            if (!VOK(h, 39)) break;
             b.key[h] = (unsigned long long)(unsigned)v << 32 | (unsigned)u;
             if (h == v) break;
             u = __ldcg(b.par + h);
@@ -313,7 +317,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
         if (i < n) {
             v = wl[i];
             const int32_t h = __ldcg(b.skip + v);
-            const unsigned long long k = __ldcg(b.key + h);
+            const unsigned long long k = VOK(h, 39) ? __ldcg(b.key + h) : ~0ull;
             const int32_t u = (int32_t)(unsigned)k;
             left = k == ~0ull || (h <= u ? v < h || v > u : v < u || v > h);
             if (left && __ldcg(b.size + v) > 1) {
@@ -453,7 +457,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_cycles(Run<OffT> r, Ext<OffT> x, 
                     if (lane_id() < max(c, 1)) {
                         const int32_t y = w + lane_id() * dir;
                         if (c > 0 || sz == 1) set_bit(r.D, y);
-                        if (y != low) b.rep[y] = low;
+                        if (y != low && VOK(y, 40)) b.rep[y] = low;
                     }
                     __syncwarp();
                     all += sz;
@@ -523,7 +527,8 @@ __device__ __forceinline__ void super_round(const Run<OffT> &r, const CycBufs &b
                         unsigned long long at = 0;
                         if (lane == 0) at = reserve(len);
                         at = __shfl_sync(kFull, at, 0);
-                        for (int j = lane; j < len; j += 32) q_out[at + j] = __ldcg(b.order + at0 + j);
+                        for (int j = lane; j < len; j += 32)
+                            if (VOK((long long)at + j, 36) && VOK(at0 + j, 37)) q_out[at + j] = __ldcg(b.order + at0 + j);
                     }
                 }
             }
@@ -597,7 +602,8 @@ __device__ __noinline__ void super_peel(const Run<OffT> &r, const Ext<OffT> &x, 
     if (!grid_sync(r.gsync, r.err)) return;
     for (int64_t i = gt; i < n; i += nt) {
         const int32_t v = L[i];
-        b.order[(int32_t)(atomicAdd(b.key + __ldcg(b.rep + v), 1ull << 32) >> 32)] = v;
+        const int32_t at = (int32_t)(atomicAdd(b.key + __ldcg(b.rep + v), 1ull << 32) >> 32);
+        if (VOK(at, 38)) b.order[at] = v;
     }
     if (!grid_sync(r.gsync, r.err)) return;
     // active edges between nodes; a node's vertices are near each other in the
@@ -640,7 +646,8 @@ __device__ __noinline__ void super_peel(const Run<OffT> &r, const Ext<OffT> &x, 
             unsigned long long at = 0;
             if (lane == 0) at = atomicAdd(qc, (unsigned long long)len);
             at = __shfl_sync(kFull, at, 0);
-            for (int j = lane; j < len; j += 32) b.q[0][at + j] = __ldcg(b.order + at0 + j);
+            for (int j = lane; j < len; j += 32)
+                if (VOK((long long)at + j, 36) && VOK(at0 + j, 37)) b.q[0][at + j] = __ldcg(b.order + at0 + j);
         }
     }
     if (!grid_sync(r.gsync, r.err)) return;
@@ -745,7 +752,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_super(Run<OffT> r, Ext<OffT> x, C
 #pragma unroll
             for (int q = 0; q < 4; ++q) far = flip ? max(far, rw[q]) : min(far, rw[q]);
         }
-        if (far != rv) {
+        if (far != rv && VOK(far, 41)) {
             atomicAdd(diff + min(rv, far), 1);
             atomicAdd(diff + max(rv, far) + 1, -1);
         }

@@ -754,6 +754,7 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
         m.q[0] = reinterpret_cast<uint32_t *>(c->qv[0]);
         m.q[1] = reinterpret_cast<uint32_t *>(c->qv[1]);
         m.cap_q = r.V;
+        m.cap_e = b.cap_e;
         m.order = reinterpret_cast<int32_t *>(m.q[1]);
         m.pos = reinterpret_cast<int32_t *>(m.val[0]);
         for (int it = 0; it < kResIts; ++it) {

@@ -71,6 +71,7 @@ struct ResBufs {
     int32_t *list[2];       // [n] vertices left
     uint32_t *q[2];         // [cap_q] changed vertices, the direction in the top bit
     int64_t cap_q;
+    int64_t cap_e;          // entries of each of adj
     int32_t *order;         // [n] vertices grouped by component (overlays q[1])
     int32_t *pos;           // [n] place of a vertex in order (overlays val[0])
 };
@@ -83,6 +84,27 @@ __device__ __forceinline__ uint32_t mix32(uint32_t h) {
     h *= 0x846ca68bu;
     h ^= h >> 16;
     return h;
+}
+
+// Entry k of one direction's lists, and of a list of vertices (checked
+// builds: the position and the id)
+template <bool CG = false>  // (CG: in L2, where entries move within a kernel or L1 gains nothing)
+__device__ __forceinline__ int32_t res_adj(const ResBufs &m, const int32_t *adj, int32_t k) {
+    if (!ICHK(k >= 0 && k < m.cap_e, 20, k)) return 0;
+    const int32_t w = CG ? __ldcg(adj + k) : adj[k];
+    return VOK(w, 21) ? w : 0;
+}
+__device__ __forceinline__ int32_t res_at(const int32_t *list, int64_t i) {
+    if (!list) return (int32_t)i;
+    if (!VOK(i, 22)) return 0;
+    const int32_t v = list[i];
+    return VOK(v, 23) ? v : 0;
+}
+
+// The vertex that a label belongs to
+__device__ __forceinline__ uint32_t res_holder(const LabelMix<32> &mix, uint32_t l) {
+    const uint32_t v = mix.holder(l);
+    return VOK((long long)v, 29) ? v : 0u;
 }
 
 // The value of a vertex: a mask of pivots while splitting (OR, 16 or 64 bits
@@ -119,7 +141,7 @@ __device__ __forceinline__ int32_t res_near(const ResBufs &m, int d, int32_t v) 
     const int32_t mine = m.old[v];
     int32_t at = v, near = 0x7fffffff;
     for (int32_t k = m.beg[d][v], e = m.end[d][v]; k < e; ++k) {
-        const int32_t w = m.adj[d][k], far = abs(m.old[w] - mine);
+        const int32_t w = res_adj(m, m.adj[d], k), far = abs(m.old[w] - mine);
         if (far < near) { near = far; at = w; }
     }
     return at;
@@ -151,7 +173,7 @@ __device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int3
     for (int u = 0; u < kResU; ++u) {
         nw[u] = own[u];
         if constexpr (K == R_MIN)
-            if (v[u] >= 0) nw[u] = min(own[u], __ldcg(val + mix.holder(own[u])));
+            if (v[u] >= 0) nw[u] = min(own[u], __ldcg(val + res_holder(mix, own[u])));
     }
     bool more = true;
     for (int step = 0; step < kResLane && more; step += 4) {
@@ -160,7 +182,7 @@ __device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int3
 #pragma unroll
         for (int u = 0; u < kResU; ++u)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) w[u][q] = b[u] + q < e[u] ? adj[b[u] + q] : -1;
+            for (int q = 0; q < 4; ++q) w[u][q] = b[u] + q < e[u] ? res_adj(m, adj, b[u] + q) : -1;
 #pragma unroll
         for (int u = 0; u < kResU; ++u) {
 #pragma unroll
@@ -178,7 +200,7 @@ __device__ __forceinline__ unsigned res_pull(const ResBufs &m, int d, const int3
                 const int l = __ffs(g) - 1;
                 const int32_t lb = __shfl_sync(kFull, b[u], l), le = __shfl_sync(kFull, e[u], l);
                 T acc = (T)__shfl_sync(kFull, nw[u], l);
-                for (int32_t k = lb + lane_id(); k < le; k += 32) acc = res_join<K>(acc, __ldcg(val + adj[k]));
+                for (int32_t k = lb + lane_id(); k < le; k += 32) acc = res_join<K>(acc, __ldcg(val + res_adj(m, adj, k)));
                 acc = res_warp_join<K>(acc);
                 if (lane_id() == l) nw[u] = acc;
             }
@@ -211,14 +233,14 @@ __device__ __forceinline__ bool res_pull_linked(const ResBufs &m, int d, int32_t
         const uint32_t far = __ldcg(link + v), to = __ldcg(link + far);
         own = __ldcg(val + v);
         nw = res_join<K>(own, __ldcg(val + far));
-        if constexpr (K == R_MIN) nw = min(nw, __ldcg(val + mix.holder(own)));
+        if constexpr (K == R_MIN) nw = min(nw, __ldcg(val + res_holder(mix, own)));
         __stcg(link + v, again ? (uint32_t)res_near(m, d, v) : to);
     }
     const int32_t c = min(e, b + kResLane);
     for (; b < c; b += 4) {
         int32_t w[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) w[q] = b + q < c ? adj[b + q] : v;
+        for (int q = 0; q < 4; ++q) w[q] = b + q < c ? res_adj(m, adj, b + q) : v;
 #pragma unroll
         for (int q = 0; q < 4; ++q) nw = res_join<K>(nw, __ldcg(val + w[q]));
     }
@@ -227,7 +249,7 @@ __device__ __forceinline__ bool res_pull_linked(const ResBufs &m, int d, int32_t
         const int l = __ffs(g) - 1;
         const int32_t lb = __shfl_sync(kFull, b, l), le = __shfl_sync(kFull, e, l);
         T acc = (T)__shfl_sync(kFull, nw, l);
-        for (int32_t k = lb + lane_id(); k < le; k += 32) acc = res_join<K>(acc, __ldcg(val + adj[k]));
+        for (int32_t k = lb + lane_id(); k < le; k += 32) acc = res_join<K>(acc, __ldcg(val + res_adj(m, adj, k)));
         acc = res_warp_join<K>(acc);
         if (lane_id() == l) nw = acc;
     }
@@ -259,7 +281,7 @@ __device__ __forceinline__ void res_push(const ResBufs &m, bool have, uint32_t e
         const int ld = (int)(le_ent >> 31);
         T *lval = reinterpret_cast<T *>(m.val[ld]);
         for (int32_t k = lb; k < le; k += 32) {
-            const int32_t w = k + lane_id() < le ? __ldcg(m.adj[ld ^ 1] + k + lane_id()) : -1;
+            const int32_t w = k + lane_id() < le ? res_adj<true>(m, m.adj[ld ^ 1], k + lane_id()) : -1;
             bool grew = false;
             if (w >= 0) {
                 T x = __ldcg(lval + w);
@@ -280,7 +302,7 @@ __device__ __forceinline__ void res_push(const ResBufs &m, bool have, uint32_t e
         T xv[4];
         unsigned grew = 0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) w[q] = b + q < e ? __ldcg(adj + b + q) : -1;
+        for (int q = 0; q < 4; ++q) w[q] = b + q < e ? res_adj<true>(m, adj, b + q) : -1;
 #pragma unroll
         for (int q = 0; q < 4; ++q) xv[q] = w[q] >= 0 ? __ldcg(val + w[q]) : mv;
 #pragma unroll
@@ -347,7 +369,7 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
             if (!((dirs >> d) & 1)) continue;
             link[d] = K == R_MIN ? m.val[d] + all : m.val[d ^ 1];  // (masks spread one way at a time)
             for (int64_t i = gt; i < n; i += nt) {
-                const int32_t v = list ? list[i] : (int32_t)i;
+                const int32_t v = res_at(list, i);
                 link[d][v] = (uint32_t)res_near(m, d, v);
             }
         }
@@ -368,7 +390,7 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
             int changed = 0;
             if (linked)
                 for (int64_t i = gt; i - threadIdx.x < n; i += nt) {
-                    const int32_t v = i < n ? (list ? list[i] : (int32_t)i) : -1;
+                    const int32_t v = i < n ? res_at(list, i) : -1;
                     for (int d = 0; d < 2; ++d)
                         if ((dirs >> d) & 1)
                             changed += res_pull_linked<K>(m, d, v, link[d], levels % kResAgain == kResAgain - 1, mix);
@@ -379,7 +401,7 @@ __device__ __forceinline__ int res_spread(const Run<int32_t> &r, const ResBufs &
 #pragma unroll
                 for (int u = 0; u < kResU; ++u) {
                     const int64_t i = i0 + u * 32 + lane_id();
-                    v[u] = i < n ? (list ? list[i] : (int32_t)i) : -1;
+                    v[u] = i < n ? res_at(list, i) : -1;
                 }
                 for (int d = 0; d < 2; ++d) {
                     if (!((dirs >> d) & 1)) continue;
@@ -521,10 +543,11 @@ __device__ __forceinline__ void res_prune(const ResBufs &m, int d, int64_t v0, i
         for (int st = 16; st; st >>= 1)
             if (__shfl_sync(kFull, incl, o + st - 1) <= k) o += st;
         const uint32_t co = __shfl_sync(kFull, c, o & 31);
-        const int32_t w = k < total ? __ldcg(adj + base + k) : -1;
+        const int32_t w = k < total ? res_adj<true>(m, adj, base + k) : -1;
         const bool keep = w >= 0 && cls(w) == co;
         const unsigned g = __ballot_sync(kFull, keep);
-        if (keep) __stcg(adj + base + out + __popc(g & lanemask_lt()), w);
+        if (keep && ICHK(base + out >= 0 && base + out < m.cap_e, 24, base + out))
+            __stcg(adj + base + out + __popc(g & lanemask_lt()), w);
         out += __popc(g);
         // the step's bits that are mine: entries [my0, incl) - k0, cut to [0, 32)
         const int32_t lo = max(0, my0 - k0), hi = min(32, incl - k0);
@@ -556,7 +579,7 @@ __device__ __forceinline__ void res_prune_one(const ResBufs &m, int32_t v, Cls c
             int32_t u[4];
             uint32_t cu[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) u[q] = k + q < e ? __ldcg(adj + k + q) : -1;
+            for (int q = 0; q < 4; ++q) u[q] = k + q < e ? res_adj<true>(m, adj, k + q) : -1;
 #pragma unroll
             for (int q = 0; q < 4; ++q) cu[q] = u[q] >= 0 ? cls(u[q]) : ~c;
 #pragma unroll
@@ -596,7 +619,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
     // ended next to nothing: one SCC, on which masks are lost
     const int64_t before = it > 1 ? (int64_t)__ldcg(x.ctl + K_RES_LEFT + it - 2) : n;
     if (it && (nl < n / kResFew || 10 * nl > 9 * before || __ldcg(x.ctl + K_RES_STOP))) {
-        for (int64_t i = gt; i < nl; i += nt) m.list[it & 1][i] = list[i];
+        for (int64_t i = gt; i < nl; i += nt) m.list[it & 1][i] = res_at(list, i);
         if (gt == 0) x.ctl[K_RES_LEFT + it] = (unsigned long long)nl;
         return;
     }
@@ -610,7 +633,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
     if (gt < 3) { chg[gt] = 0ull; qc[gt] = 0ull; }
     for (int64_t i = gt; i < nl; i += nt) {
         int32_t root, size;
-        const int32_t v = list ? list[i] : (int32_t)i;
+        const int32_t v = res_at(list, i);
         if (it == 0) {  // the WCCs
             root = m.parent[m.old[v]];
             size = m.wsize[root];
@@ -630,7 +653,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
         unsigned short *v16 = reinterpret_cast<unsigned short *>(m.val[d]);
         if (gt == 0) { chg[s == 2 ? 0 : s + 1] = 0ull; qc[s == 2 ? 0 : s + 1] = 0ull; }
         for (int64_t i = gt; i < nl; i += nt) {
-            const int32_t v = list ? list[i] : (int32_t)i;
+            const int32_t v = res_at(list, i);
             const uint32_t h = mix32((uint32_t)v * 16u + (uint32_t)(4 * it + k) + 1u);
             const int shift = max(kResSplitShift, (int)(m.cls[v] >> 27) - bits * (it ? 1 : k + 1));
             const bool pivot = (h >> (32 - shift)) == 0u;
@@ -650,7 +673,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
             break;
         }
         for (int64_t i = gt; i < nl; i += nt) {
-            const int32_t v = list ? list[i] : (int32_t)i;
+            const int32_t v = res_at(list, i);
             const uint32_t c = m.cls[v];
             const unsigned long long y = wide ? __ldcg(v64 + v) : (unsigned long long)__ldcg(v16 + v);
             m.cls[v] = (mix32(c ^ mix32((uint32_t)y ^ mix32((uint32_t)(y >> 32)))) & kResHash) | (c & ~kResHash);
@@ -662,7 +685,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
                     res_prune(m, 1, g * 32, n, cls);
                 }
             else
-                for (int64_t i = gt; i < nl; i += nt) res_prune_one(m, list[i], cls);
+                for (int64_t i = gt; i < nl; i += nt) res_prune_one(m, res_at(list, i), cls);
         };
         // an entry led to the same class before, so 16-bit masks tell where it
         // leads now: half the words to gather (21 M vertices, 84 MB of class words: 1.4-1.9 ms a round)
@@ -679,19 +702,19 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
     int32_t *first = reinterpret_cast<int32_t *>(m.val[1]);  // [tiles]: start of the first component in each tile
     const int64_t tiles = nl / kTileT + 1;
     for (int64_t i = gt; i < nl; i += nt) {
-        const int32_t v = list ? list[i] : (int32_t)i;
+        const int32_t v = res_at(list, i);
         uf[v] = v;
         cnt[v] = 0;
     }
     for (int64_t i = gt; i < tiles; i += nt) first[i] = 0x7fffffff;
     if (!grid_sync(r.gsync, r.err)) return;
     for (int64_t i = gt; i < nl; i += nt) {
-        const int32_t v = list ? list[i] : (int32_t)i;
-        for (int32_t k = m.beg[0][v], e = m.end[0][v]; k < e; ++k) uf_hook(uf, v, __ldcg(m.adj[0] + k));
+        const int32_t v = res_at(list, i);
+        for (int32_t k = m.beg[0][v], e = m.end[0][v]; k < e; ++k) uf_hook(uf, v, res_adj<true>(m, m.adj[0], k));
     }
     if (!grid_sync(r.gsync, r.err)) return;
     for (int64_t i = gt; i - threadIdx.x < nl; i += nt) {
-        const int32_t v = i < nl ? (list ? list[i] : (int32_t)i) : -1;
+        const int32_t v = i < nl ? res_at(list, i) : -1;
         const int32_t root = v >= 0 ? uf_root(uf, v) : -1;
         if (v >= 0) uf[v] = root;
         const unsigned grp = __match_any_sync(kFull, root);
@@ -699,7 +722,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
     }
     if (!grid_sync(r.gsync, r.err)) return;
     for (int64_t i = gt; i - threadIdx.x < nl; i += nt) {  // a run of m.order for each component that fits a tile
-        const int32_t v = i < nl ? (list ? list[i] : (int32_t)i) : -1;
+        const int32_t v = i < nl ? res_at(list, i) : -1;
         const bool root = v >= 0 && uf[v] == v;
         const int32_t c = root ? __ldcg(cnt + v) : 0;
         const bool small = c > 0 && c <= kTileT, mid = c > kTileT && c <= kTileV;
@@ -721,8 +744,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
         } else if (mid) {
             b = (int32_t)(nl - (int64_t)atomicAdd(work + W_BACK, (unsigned long long)c)) - c;
             const unsigned long long q = atomicAdd(work + W_MID, 1ull);
-            m.q[0][2 * q] = (uint32_t)b;  // (a mid component has over two vertices: q fits)
-            m.q[0][2 * q + 1] = (uint32_t)c;
+            if (VOK((long long)(2 * q + 1), 28)) {  // (a mid component has over two vertices: q fits)
+                m.q[0][2 * q] = (uint32_t)b;
+                m.q[0][2 * q + 1] = (uint32_t)c;
+            }
         }
         if (root) base[v] = b;
     }
@@ -731,12 +756,12 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
         bool big = false;
         int32_t v = 0;
         if (i < nl) {
-            v = list ? list[i] : (int32_t)i;
+            v = res_at(list, i);
             const int32_t root = uf[v], b = base[root];
             big = b < 0;
             if (!big) {
                 const int32_t at = b + atomicSub(cnt + root, 1) - 1;
-                m.order[at] = v;
+                if (VOK(at, 25)) m.order[at] = v;
                 m.pos[v] = at;
             }
         }
@@ -786,8 +811,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Run<int32_t> r, Ext<i
         __syncthreads();
         const int n = t.count, start = t.start;
         if (n < 0) break;
-        if (n == 0) continue;
-        for (int i = tid; i < n; i += kTileThreads) t.f[i] = m.old[m.order[start + i]];
+        if (n == 0 || !ICHK(n <= kTileV && start >= 0, 27, ((long long)start << 32) | n)) continue;
+        for (int i = tid; i < n; i += kTileThreads) t.f[i] = m.old[res_at(m.order, start + i)];
         for (int i = tid; i < kTileV / 32; i += kTileThreads) t.dead[i] = 0u;
         tile_sort(t, n);
         int32_t e0[kTilePer];  // the list of each of my vertices
@@ -827,10 +852,14 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tiles(Run<int32_t> r, Ext<i
             for (int k = 0; k < d; k += 4) {
                 int32_t w[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) w[q] = k + q < d ? __ldcg(m.adj[1] + e0[u] + k + q) : -1;
+                for (int q = 0; q < 4; ++q) w[q] = k + q < d ? res_adj<true>(m, m.adj[1], e0[u] + k + q) : -1;
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (w[q] >= 0) t.adj[o + k + q] = (uint16_t)t.f[__ldcg(m.pos + w[q]) - start];
+                for (int q = 0; q < 4; ++q) {
+                    if (w[q] < 0) continue;
+                    const int p = __ldcg(m.pos + w[q]) - start;
+                    if (ICHK(p >= 0 && p < n && o + k + q < kTileE, 26, ((long long)p << 32) | (o + k + q)))
+                        t.adj[o + k + q] = (uint16_t)t.f[p];
+                }
             }
         }
         tile_solve(t, n, r, done, sccs);
@@ -859,7 +888,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
         if (gt == 0) left[(k + 1) % 3] = 0ull;
         const LabelMix<32> mix(k);
         for (int64_t i = gt; i < nl; i += nt) {
-            const int32_t v = list[i];
+            const int32_t v = res_at(list, i);
             m.val[0][v] = m.val[1][v] = mix.label((uint32_t)v);
             m.mn[v] = 0x7fffffff;
             m.size[v] = 0;
@@ -867,10 +896,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
         if (!grid_sync(r.gsync, r.err)) return;
         if (res_spread<R_MIN>(r, m, chg, qc, x.ctl + K_LARGE, list, nl, 3, s, sm, false, mix) != 1) return;
         for (int64_t i = gt; i < nl; i += nt) {
-            const int32_t v = list[i];
+            const int32_t v = res_at(list, i);
             const uint32_t f = __ldcg(m.val[0] + v);
             if (f == __ldcg(m.val[1] + v)) {
-                const uint32_t p = mix.holder(f);
+                const uint32_t p = res_holder(mix, f);
                 atomicMin(m.mn + p, m.old[v]);
                 atomicAdd(m.size + p, 1);
             }
@@ -881,14 +910,14 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
             bool keep = false;
             int32_t v = 0;
             if (i < nl) {
-                v = list[i];
+                v = res_at(list, i);
                 const uint32_t f = __ldcg(m.val[0] + v), b = __ldcg(m.val[1] + v);
                 keep = f != b;
                 if (keep) {
                     m.cls[v] = mix32(f ^ mix32(b)) & 0x7fffffffu;
                 } else {
                     const int32_t ov = m.old[v];
-                    r.label[ov] = __ldcg(m.mn + mix.holder(f));
+                    r.label[ov] = __ldcg(m.mn + res_holder(mix, f));
                     r.cls[ov] = CLS_MICE;
                     clear_bit(r.A, ov);
                     m.cls[v] = kResDead;
@@ -929,7 +958,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_resolve(Run<int32_t> r, Ext<int32
         }
         list = next;
         nl = nn;
-        for (int64_t i = gt; i < nl; i += nt) res_prune_one(m, list[i], [&](int32_t w) { return __ldcg(m.cls + w); });
+        for (int64_t i = gt; i < nl; i += nt) res_prune_one(m, res_at(list, i), [&](int32_t w) { return __ldcg(m.cls + w); });
         if (!grid_sync(r.gsync, r.err)) return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) r.counters[C_COLOR_ROUNDS] = (unsigned long long)rounds;

@@ -99,7 +99,8 @@ __device__ __forceinline__ void small_list(SmallSmem &s, const Run<OffT> &r, int
     const OffT *beg = d ? r.bw_beg : r.fw_beg;
     const int64_t n = ld_off(beg, v + 1) - ld_off(beg, v);
     const int c = n <= kSmallLane ? 0 : n <= kSmallHub ? 1 : 2;
-    s.list[c][atomicAdd(&s.n[c], 1)] = (uint32_t)v | (uint32_t)d << 31;
+    const int at = atomicAdd(&s.n[c], 1);
+    if (ICHK(at < kSmallOwn * 64 + kSmallQ, 42, at)) s.list[c][at] = (uint32_t)v | (uint32_t)d << 31;
 }
 
 // The vertices of the own words m[d] for the directions of `dirs` (bit 0:

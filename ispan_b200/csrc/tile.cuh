@@ -114,13 +114,21 @@ __device__ __forceinline__ void tile_sort(T &t, int n) {
     __syncthreads();
 }
 
+// entry k of the tile's lists (checked builds: the position and the id)
+template <typename T>
+__device__ __forceinline__ int tile_adj(const T &t, int k) {
+    if (!ICHK(k >= 0 && k < T::kE, 30, k)) return 0;
+    const int w = t.adj[k];
+    return ICHK(w < T::kV, 31, w) ? w : 0;
+}
+
 // i's links anew: the descendant nearest by id, and i as that one's ancestor
 // (of several, any).
 template <typename T>
 __device__ __forceinline__ void tile_link(T &t, int i) {
     int near = 0xffff, at = i;
     for (int k = t.off[i], z = k + t.len[i]; k < z; ++k) {
-        const int w = t.adj[k], far = abs(w - i);
+        const int w = tile_adj(t, k), far = abs(w - i);
         if (far < near && far) { near = far; at = w; }
     }
     t.link[1][i] = (uint16_t)at;
@@ -133,6 +141,7 @@ __device__ __forceinline__ void tile_link(T &t, int i) {
 // done and sccs.  Ends with a barrier.
 template <typename T, typename RunT>
 __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &done, int64_t &sccs) {
+    if (!ICHK(n >= 0 && n <= T::kV, 32, n)) return;
     constexpr int kPer = T::kPer;
     const int tid = threadIdx.x;
     unsigned mine = 0;  // my vertices not solved yet
@@ -183,7 +192,7 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
                 int32_t bv = min(min(b0, b[mix.holder(b0)]), b[ld]);
                 const int o = t.off[i], z = o + t.len[i];
                 for (int k = o; k < z; ++k) {
-                    const int w = t.adj[k];
+                    const int w = tile_adj(t, k);
                     if (f[w] > fv) { atomicMin(&t.f[w], fv); ch = 1; }
                     bv = min(bv, b[w]);
                 }
@@ -238,6 +247,7 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
             if (!((sol >> u) & 1u)) continue;
             const bool root = (roots >> u) & 1u;
             const int32_t lab = root ? t.f[i] : t.f[mix.holder(t.f[i])], ov = orig[u];
+            if (!VOK(ov, 33)) continue;
             r.label[ov] = lab;
             r.cls[ov] = CLS_MICE;
             clear_bit(r.A, ov);
@@ -257,7 +267,7 @@ __device__ __forceinline__ void tile_solve(T &t, int n, const RunT &r, int64_t &
             const int o = t.off[i], z = o + t.len[i];
             int q = o;
             for (int k = o; k < z; ++k) {
-                const int w = t.adj[k];
+                const int w = tile_adj(t, k);
                 if (!((t.dead[w >> 5] >> (w & 31)) & 1u) && t.f[w] == fv && t.b[w] == bv) t.adj[q++] = (uint16_t)w;
             }
             t.len[i] = (uint16_t)(q - o);
