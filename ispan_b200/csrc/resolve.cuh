@@ -47,11 +47,12 @@ constexpr int kResIts = 3;             // times k_split and k_tiles run
 constexpr int64_t kResFew = 16;        // fewer vertices left than 1 / 16: no more splitting (a time takes ~1.5 ms even
                                        // for few; the labelling rounds of 18,000 vertices 0.5 ms)
 // Width of the masks: 64 bits (three rounds) while their array stays in L2,
-// 48 MB; then 16 bits (four rounds) up to 64 MB; beyond, every gather is a
-// DRAM access whatever its width, and 64 bits split most.  (21 M vertices:
-// 34 ms a first round with 64 bits, 19 with 32, 9-11 with 16.)
+// 48 MB; beyond, 16 bits (four rounds): a gather is then a DRAM access more
+// often than not, and a dense pass takes the time of its traffic.  (21 M
+// vertices: 34 ms a first round with 64 bits, 19 with 32, 9-11 with 16.  42 M
+// and 84 M, a call on a web graph: 347-382 and 826-914 ms with 64 bits, 297-350
+// and 697-845 with 16.)
 constexpr int64_t kResWideN = 6 << 20;
-constexpr int64_t kResNarrowN = 32 << 20;
 constexpr int64_t kResSparse = 16;     // a pass that changed at most 1 / 16 of the vertices ends the dense passes
                                        // (a listed vertex costs ~0.17 ns to push, a dense pass ~0.01-0.017 ns a vertex);
                                        // more listed ones than that begin them again
@@ -625,7 +626,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_split(Run<int32_t> r, Ext<int32_t
     }
     // masks as wide as their array stays in L2 (gathers from both dies: about
     // half of its 126 MB): wider ones split more per round
-    const bool wide = n <= kResWideN || n > kResNarrowN;
+    const bool wide = n <= kResWideN;
     const int bits = wide ? 6 : 4;  // log2 of the pivots per class aimed at
     // (what k_super left of the large WCCs has mostly fallen apart: its
     // components first)
