@@ -60,7 +60,11 @@ typedef struct {
  * below |worklist| / beta or the level exceeds gamma.  theta is the
  * reference's trim stop ratio; the peel here runs to a fixpoint, so theta is
  * accepted and recorded only.  Zero fields take the reference defaults
- * 30/200/10/0.1 (src/bash_one.sh:4). */
+ * 30/200/10/0.1 (src/bash_one.sh:4).  A graph of at most 65,536 vertices and
+ * 4,194,304 edges is searched inside one cluster of 16 CTAs by switches of its
+ * own: alpha, beta and gamma act on it only where the stage kernels run
+ * (ISPAN_F_STAGE_TIMES, ISPAN_F_EXACT_STATS, tiny_residual, or a device on
+ * which no such cluster fits). */
 typedef struct {
     int32_t alpha, beta, gamma;
     double theta;
@@ -68,8 +72,10 @@ typedef struct {
 } ispan_params;
 
 #define ISPAN_F_LABELS_ON_DEVICE 1u /* labels_out is device memory */
-#define ISPAN_F_NO_GRAPH 2u         /* launch stages directly, no CUDA graph */
-#define ISPAN_F_STAGE_TIMES 4u      /* record per-stage device times */
+#define ISPAN_F_NO_GRAPH 2u         /* launch stages directly, no CUDA graph (otherwise the first run
+                                       of an input launches directly, the second in a row captures) */
+#define ISPAN_F_STAGE_TIMES 4u      /* record per-stage device times, of the stage kernels: small
+                                       graphs take them with this flag and one cluster without */
 #define ISPAN_F_NO_L2_WINDOW 8u     /* no persisting L2 window over the status maps */
 #define ISPAN_F_VALIDATE 16u        /* check a device-resident CSR before the run
                                        (host CSRs are always checked) */
@@ -85,7 +91,12 @@ typedef struct {
  * Finer slots without a reference counterpart: 11 colouring of the large
  * WCCs (part of 10), 12 second trim-1 peel, 14 residual worklist after the
  * pivot SCCs, 15 first trim-1 peel (12, 14, 15 are parts of 4).
- * Milliseconds of device time. */
+ * Milliseconds of device time.  fw_levels and bw_levels count the searches'
+ * rounds: one level each in the synchronous modes, several where a search runs
+ * asynchronously or inside one cluster, so they differ between the routes a
+ * small graph may take (see ispan_params); color_rounds counts the splitting and
+ * labelling or colouring rounds of the large WCCs, trim_rounds the rounds of the
+ * peels. */
 typedef struct {
     double stage_ms[16];
     int64_t scc_count;        /* number of SCCs (no phantom vertex, unlike Q1) */
@@ -122,7 +133,12 @@ int64_t ispan_ctx_bytes(int64_t max_V, int64_t max_E);
 /* Launch tunables of a context, chosen per graph-shape class by the
  * autotuner (ispan_b200/autotune.py).  They change scheduling only, never
  * labels.  Zero fields take the defaults.  The reference's only knobs are
- * alpha/beta/gamma/theta (src/scc_main.cpp:16-25); these have no counterpart. */
+ * alpha/beta/gamma/theta (src/scc_main.cpp:16-25); these have no counterpart.
+ * async_*, bfs_ctas_per_sm and pair_searches act on graphs beyond 65,536 vertices
+ * or 4,194,304 edges (smaller ones: as alpha, beta and gamma).  color_levels and
+ * color_pivots act where the large WCCs have no compact graph: they are fewer
+ * than 65,536 vertices or more than a quarter of the graph's, their edges do not
+ * fit its scratch, or color_compact is off. */
 typedef struct {
     int64_t async_v;          /* a search goes asynchronous below this many frontier vertices (65536) */
     int64_t async_e;          /* ... and this many frontier edges (262144) */
@@ -131,11 +147,13 @@ typedef struct {
     int32_t color_levels;     /* colouring large WCCs: a warp works up to 4 * color_levels chunks of 32
                                  frontier entries per grid round before handing the rest back (32) */
     int32_t color_pivots;     /* about this many pivots in the first colouring round; doubles per round (1024) */
-    int32_t color_compact;    /* colour the large WCCs on a compact copy of their subgraph (dense ids,
-                                 only their edges among themselves): 1 on, -1 off (0: default, on) */
+    int32_t color_compact;    /* split and label the large WCCs on a compact copy of their subgraph (dense
+                                 ids, only their edges among themselves): 1 on, -1 off, they are coloured
+                                 on the input graph (0: default, on) */
     int32_t pair_searches;    /* run the forward and backward giant searches at the same time (the
                                  backward one over all active vertices; pivot SCC = both sets'
-                                 intersection): 1 on, -1 off, 0 on for graphs of at most 2^20 vertices */
+                                 intersection): 1 on, -1 off, 0 on for graphs of at most 2^20 vertices
+                                 (in one cluster always) */
     int32_t tiny_residual;    /* solve a residual of at most 1024 vertices (and 4096 edges among them per
                                  direction) after the giant SCC in one CTA, skipping the later stage
                                  kernels: 1 on (0: default, off) */
@@ -144,7 +162,7 @@ typedef struct {
                                  kernel's tail: -1 off (0: default, on) */
 } ispan_tuning;
 
-/* NULL restores the defaults; the next run re-captures its CUDA graph. */
+/* NULL restores the defaults; captured CUDA graphs are dropped. */
 int ispan_ctx_set_tuning(ispan_ctx *ctx, const ispan_tuning *t);
 /* the values in effect (defaults filled in; bfs_ctas_per_sm 0 = occupancy limit) */
 int ispan_ctx_get_tuning(ispan_ctx *ctx, ispan_tuning *t);

@@ -9,7 +9,10 @@ warp does per grid round when colouring large WCCs (color_levels: up to
 4 * color_levels chunks of 32 frontier entries; less balances the CTAs, more
 saves grid barriers) and the pivots of the colouring's first round
 (color_pivots).  None of them changes a label; they
-only move time between stages.
+only move time between stages.  The last two act only where the large WCCs have
+no compact graph (small or dense remainders).  None acts on a graph that runs in
+one cluster (:func:`in_one_cluster`): runs with stage times take the stage
+kernels there, plain runs do not, so such a workload is not tuned.
 
 Method: coordinate descent from the defaults over a small grid per
 parameter, two passes, each candidate timed as the median of several runs on
@@ -18,7 +21,7 @@ mice stages.
 The winners are stored per shape class in ``tuning_table.json`` beside this
 file; :func:`apply` looks a graph's class up and sets the context.
 
-    python -m ispan_b200.autotune --workloads social,web:0.1,rmat16,batch:0.05
+    python -m ispan_b200.autotune --workloads social,web:0.1,rmat17,batch:0.05
 """
 from __future__ import annotations
 
@@ -56,11 +59,16 @@ def shape_class(V: int, E: int, nseg: int = 1) -> str:
     return f"{size}-{deg}-{'batch' if nseg > 1 else 'one'}"
 
 
+def in_one_cluster(V: int, E: int) -> bool:
+    """Whether a plain run takes the one-cluster kernel, on which no tunable acts
+    (the sizes of ispan_b200/csrc/small.cuh)."""
+    return V <= 1 << 16 and E <= 1 << 22
+
+
 def load_table(path: str = TABLE) -> dict:
     if os.path.exists(path):
         with open(path) as f:
             return json.load(f)
-    return {"classes": {}}
     return {"classes": {}}
 
 
@@ -132,8 +140,8 @@ def _workload(spec: str):
         return gen.social(seed=1, scale=scale), None
     if name == "web":
         return gen.web(seed=1, scale=scale), None
-    if name == "rmat16":
-        return gen.rmat(16, 16, 1), None
+    if name.startswith("rmat"):
+        return gen.rmat(int(name[4:]), 16, 1), None
     if name == "batch":
         g = gen.batch(nseg=max(2, int(4096 * scale)), seed=1)
         return g, g.vbase
@@ -145,7 +153,7 @@ def main():
 
     from . import Context
     ap = argparse.ArgumentParser()
-    ap.add_argument("--workloads", default="social,web:0.1,rmat16,batch:0.05")
+    ap.add_argument("--workloads", default="social,web:0.1,rmat17,batch:0.05")
     ap.add_argument("--reps", type=int, default=5)
     ap.add_argument("--passes", type=int, default=2)
     ap.add_argument("--out", default=TABLE)
@@ -156,6 +164,10 @@ def main():
         nseg = 1 if vbase is None else len(vbase) - 1
         cls = shape_class(g.V, g.E, nseg)
         print(f"{spec}: V={g.V} E={g.E} class {cls}", flush=True)
+        if in_one_cluster(g.V, g.E):
+            print("  runs in one cluster: no tunable acts", flush=True)
+            g.free()
+            continue
         ctx = Context(g.V, g.E)
         lab = torch.empty(max(g.V, 1), dtype=torch.int32, device="cuda")
         fb, fa, bb, ba = g.ptrs

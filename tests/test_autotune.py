@@ -60,3 +60,30 @@ def test_descent_keeps_only_clear_gains():
     best, ms, dms = AT.tune(ctx, run, passes=2, reps=1, log=lambda *_: None)
     assert (best["alpha"], best["beta"], best["async_deg"]) == (100, 1000, 64)
     assert ms == 10.0 and dms == 13.0
+
+
+def test_small_graphs_are_not_tuned(monkeypatch, tmp_path, capsys):
+    """What runs in one cluster is not tuned by the stage kernels' times: the
+    workload is passed over and the table keeps what it holds."""
+    import re
+    import os
+    src = open(os.path.join(AT.HERE, "csrc", "small.cuh")).read()
+    for name, value in (("kSmallV", 1 << 16), ("kSmallE", 1 << 22)):
+        got = re.search(name + r" = (\d+) << (\d+);", src)
+        assert int(got[1]) << int(got[2]) == value
+    assert AT.in_one_cluster(1 << 16, 1 << 22)
+    assert not AT.in_one_cluster((1 << 16) + 1, 10) and not AT.in_one_cluster(10, (1 << 22) + 1)
+
+    class Graph:
+        V, E = 1 << 16, 955_058
+
+        def free(self):
+            self.freed = True
+
+    g = Graph()
+    out = tmp_path / "t.json"
+    monkeypatch.setattr(AT, "_workload", lambda spec: (g, None))
+    monkeypatch.setattr("sys.argv", ["autotune", "--workloads", "rmat16", "--out", str(out)])
+    AT.main()
+    assert g.freed and not out.exists()
+    assert "one cluster" in capsys.readouterr().out
