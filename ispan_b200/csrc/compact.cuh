@@ -16,7 +16,7 @@
 //                               degrees there are scanned); each pair is one block of 2 V
 // so the random accesses of the rounds fall on n words instead of V, and no
 // edge check lands on a vertex outside.  The graph is built only when
-// each direction's edges fit the adjacency arrays (at most V entries, int32
+// each direction's edges fit the adjacency arrays (twice the context's vertices, int32
 // offsets); otherwise K_CMP_OK stays 0 and k_color runs on the input graph.  Membership is the active map A: at this point exactly the vertices
 // of the large WCCs are active.  The fill kernel reads only the offsets, so
 // the in-adjacency may overwrite the degree arrays.
@@ -26,16 +26,18 @@
 namespace ispan {
 
 constexpr int kScanBlocks = 1024;  // blocks of the offset scans (at most; one CTA scans their sums)
-constexpr int64_t kCmpMin = 1 << 16;  // fewer colouring vertices than this: no compact graph (the
-                                      // input graph's colour words of so few vertices stay in L2)
+constexpr int64_t kCmpMin = 1 << 16;  // fewer large-WCC vertices than this: no compact graph (the input graph's
+                                      // colour words of so few vertices stay in L2; set against the colouring
+                                      // rounds, not measured against the splitting)
 
 constexpr int64_t kCmpMinRest = 1 << 10;
 
-// Whether the compact graph is worth building: enough colouring vertices,
+// Whether the compact graph is worth building: enough large-WCC vertices,
 // and spread thinly over the id range (at most a quarter of it).  Where they
 // are dense -- a batch, whose graphs are contiguous id ranges -- the input
 // graph's words and lists are already local, and measured on the batched
-// workload the build cost more than the rounds gained.
+// workload the build cost more than the colouring rounds gained by it (whether
+// the splitting rounds gain more than it costs there is not measured).
 // What k_super left (`rest`) has mostly fallen apart into components for
 // tiles: worth it from far fewer (64 K of a batch: 6.7 ms of colouring).
 __device__ __forceinline__ bool cmp_wanted(int64_t n, int64_t V, const unsigned long long *ctl) {

@@ -33,7 +33,7 @@
 //
 // A batch of 512 graphs (82 M vertices, 42 M residual), one B200: colouring
 // 250 ms of a run's 298; k_cycles 3.0 ms (list reads 2.0, the rest latency of
-// walks) and k_super 3.5 ms (one edge pass, a scan, the labels), a run 37 ms.
+// walks) and k_super 3.5 ms (one edge pass, a scan, the labels), a run 27-35 ms.
 // With the peel alone instead of the spans 32 ms and 18 ms for what rings in
 // pieces kept from it.
 #pragma once

@@ -9,9 +9,8 @@
 // permitted.  For them this entry point keeps its scratch in a file-scope
 // device array of fixed size, so a call only launches one kernel.
 //
-// The kernel is the serial Tarjan of k_local_scc (stages.cuh) run by one
-// thread of one CTA over the whole graph, with its per-vertex stacks in the
-// static scratch instead of shared memory; the other threads initialise the
+// The kernel is an iterative Tarjan run by one thread of one CTA over the
+// whole graph, with its per-vertex stacks in the static scratch; the other threads initialise the
 // scratch.  Labels are the minimum vertex id of each SCC, as from
 // ispan_scc_run.  The kernel first checks the graph (offsets monotone from 0
 // to E, ids in [0, V)) and answers a malformed one with -1 labels, so a bad

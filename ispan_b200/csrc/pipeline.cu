@@ -1263,7 +1263,8 @@ struct HostCopy {
 // one thread, ~12 GB/s, a quarter of what the bus takes.  Here kStageThreads
 // threads fill pinned pieces, two each, and enqueue them on the run's stream;
 // all have returned, and the sources are read, when this does.  Measured for
-// 166 MB (four arrays): a call on a web graph of 3.5 M vertices 21 -> 11 ms.  False:
+// 166 MB (four arrays): a call on a web graph of 3.5 M vertices 20-24 ms by the
+// driver, 11.2-12.8 so.  False:
 // nothing was copied (pinned sources, few bytes, no staging memory or threads).
 static bool copy_staged(ispan_ctx *c, const HostCopy *cp, int n, cudaError_t &err) {
     size_t total = 0;
@@ -1279,7 +1280,7 @@ static bool copy_staged(ispan_ctx *c, const HostCopy *cp, int n, cudaError_t &er
     if (total < kStageMin || c->stage_failed || std::thread::hardware_concurrency() < 4) return false;
     if (!c->h_stage) {
         // a context's first such call does without: pinning the pieces can cost
-        // it more (5-60 ms) than it gains
+        // it more than it gains (8 MB alone: 3.6 to 19 ms, once 104)
         if (!c->stage_again) {
             c->stage_again = true;
             return false;

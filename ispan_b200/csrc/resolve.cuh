@@ -29,11 +29,12 @@
 // no atomics), until few vertices change; those are listed and push on,
 // level by level.
 //
-// What bounds it: while the gathered array stays in L2, a dense pass runs at
-// one L2 sector per edge (0.28 ms for 48 M entries); beyond about half of the
-// L2 each gather is a DRAM access (with 64-bit masks on 21 M vertices, 168
-// MB, a pass took 1.3 ms, with 32-bit ones 0.53).  In the tails a level's
-// latency counts.  Web-shaped graphs, colouring stage before and now, one
+// What bounds it: random sectors of L2 while the gathered array stays there
+// (2.1 M vertices: k_split reads 20 GB of sectors at 3.7 TB/s, levels included,
+// for 1 GB of DRAM traffic; a dense pass over 48 M entries 0.28 ms); beyond
+// about half of the L2 the gathers' DRAM traffic (with 64-bit masks on 21 M
+// vertices, 168 MB, a pass took 1.3 ms, with 32-bit ones 0.53).  In the tails a
+// level's latency counts.  Web-shaped graphs, colouring stage before and now, one
 // B200: 7 M vertices (1.1 M here) 10.0 and 5.3 ms, 140 M vertices (21 M
 // here) 244 and 85 ms.
 #pragma once

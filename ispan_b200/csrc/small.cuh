@@ -12,9 +12,9 @@
 // level ends with two cluster barriers.  The edge lists are the only global
 // reads (4 MB a direction on scale 16: about 2 us over 16 SMs).  Bound by the
 // cluster's meetings (two a level, ~1 us each) and by the latency of list
-// reads between them.  Measured, a call: R-MAT scale 10 127 -> 74 us, scale
-// 16 150 -> 105, 23 planted-cycle graphs of 100 to 5,000 930 -> 846 (the
-// kernel itself: 32 and 66 us on the R-MAT graphs).
+// reads between them.  Measured, a call, by the stage kernels and so: R-MAT scale
+// 10 115 and 70-74 us, scale 16 150 and 104 (the kernel itself: 32 and 66 us);
+// 23 planted-cycle graphs of 100 to 5,000 (0.5-0.63 ms now) gained 0.08 ms.
 // If nothing is left after the peel, the labels are written here too;
 // otherwise the stage kernels go on from the peel's lists.
 //

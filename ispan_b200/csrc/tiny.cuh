@@ -17,8 +17,7 @@
 //      thread per vertex, claims by an atomic on a shared bitmap;
 //   4. trim-1 again;
 //   5. the rest: weakly connected components (statistics, as the WCC
-//      stage counts them) and an iterative Tarjan, as k_local_scc does for
-//      a small WCC.
+//      stage counts them) and an iterative Tarjan by one thread.
 // Labels are the minimum member id, classes as the stage kernels set them,
 // counters and histogram entries as they record them, and every vertex
 // leaves the active map.  It then sets K_TINY, and the later stage kernels
@@ -297,7 +296,7 @@ __global__ void __launch_bounds__(kBlock) k_tiny_residual(Run<OffT> r, Ext<OffT>
         __syncthreads();
         if (!s.flag) break;
     }
-    // Tarjan (one thread, as k_local_scc) over the live vertices
+    // Tarjan (one thread) over the live vertices
     if (t == 0) {
         int nwcc = 0, nmice = 0, nscc = 0;
         for (int i = 0; i < n; ++i) {
