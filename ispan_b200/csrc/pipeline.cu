@@ -196,7 +196,8 @@ struct ispan_ctx {
 
     // the backward search's stream when the searches run at the same time
     cudaStream_t stream2 = nullptr;
-    // captures of the conditional parts of the graph, the inner one second
+    // captures of the conditional parts of the graph, the inner one second (made
+    // for the first capture)
     cudaStream_t stream_if[2] = {nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     bool small_fits = false;    // k_small's cluster can be resident
@@ -863,7 +864,8 @@ static void l2_window(ispan_ctx *c, bool on) {
         v.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
     }
     for (cudaStream_t t : {c->stream, c->stream_if[0], c->stream_if[1]})
-        if (cudaStreamSetAttribute(t, cudaStreamAttributeAccessPolicyWindow, &v) != cudaSuccess) cudaGetLastError();
+        if ((t == c->stream || t) && cudaStreamSetAttribute(t, cudaStreamAttributeAccessPolicyWindow, &v) != cudaSuccess)
+            cudaGetLastError();
 }
 
 template <typename OffT>
@@ -937,7 +939,13 @@ static int run_t(ispan_ctx *c, int64_t V, int64_t E, int32_t nseg, const OffT *f
                 gx = nullptr;
             }
             cudaGraph_t g = nullptr;
-            cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+            cudaError_t e = cudaSuccess;
+            if (!c->stream_if[1]) {
+                for (cudaStream_t &t : c->stream_if)
+                    if (e == cudaSuccess && !t) e = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking);
+                if (l2win) l2_window(c, true);
+            }
+            if (e == cudaSuccess) e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
                 cudaError_t e2 = enqueue<OffT>(c, r, x, ev_on, true);
                 e = cudaStreamEndCapture(c->stream, &g);
@@ -1730,8 +1738,6 @@ int ispan_ctx_create(int device, int64_t max_V, int64_t max_E, ispan_ctx **out) 
     if (!rc && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) rc = ISPAN_ERR_CUDA;
     c->own_stream = true;
     if (!rc && cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking) != cudaSuccess) rc = ISPAN_ERR_CUDA;
-    for (int i = 0; i < 2; ++i)
-        if (!rc && cudaStreamCreateWithFlags(&c->stream_if[i], cudaStreamNonBlocking) != cudaSuccess) rc = ISPAN_ERR_CUDA;
     if (!rc && (cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess))
         rc = ISPAN_ERR_CUDA;
