@@ -380,6 +380,7 @@ struct AsyncSmem {
     int32_t lq[2][kLQ];
     int cnt[2];
     int flush;  // hand the local frontier back to the grid at the next level
+    int linked[2];  // a vertex of the level led to the id next to it, by the level's parity
 };
 
 constexpr int kAsyncFlush = kLQ / 2;  // a CTA's local frontier above this is work for the whole grid
@@ -391,19 +392,24 @@ constexpr int kAsyncFlush = kLQ / 2;  // a CTA's local frontier above this is wo
 // or path of consecutive ids one level goes 15 vertices far; a level is five
 // dependent reads (offsets, list, visit map, degrees, ~3 us) whatever it
 // reaches.  Only where the CTA's frontier is at most kChainN vertices: a wider
-// one keeps a lane per vertex.
+// one keeps a lane per vertex; and after kChainMisses levels without such a link
+// every kChainRetry-th level only (a ring of 300,000 with shuffled ids: 492 ms
+// without looking ahead, 524 at every level, 507 so; one of 1,000,000 with
+// consecutive ids 1,451, 209 and 215).
 // (97 separate graphs, rings of up to 1,000: the async rounds of the two
 // searches 1,570 and 880 us by single steps, 850 and 130 so.)
 constexpr int kChainN = 2 * kWarps;
+constexpr int kChainMisses = 8, kChainRetry = 32;
 template <typename OffT, int DIR, typename Expand>
 __device__ __forceinline__ void async_chain(const Run<OffT> &r, const BfsDir<OffT, DIR> &d, int32_t v, int32_t *qvn,
                                             int64_t *qen, int32_t *qcn, unsigned long long *pk_next, int64_t &nvis,
-                                            int64_t &msum_next, Expand expand) {
+                                            int64_t &msum_next, int &linked, Expand expand) {
     const int lane = lane_id();
     const int64_t v0 = ld_off(d.xbeg, v), v1 = ld_off(d.xbeg, v + 1);
     const int32_t w0 = v0 + lane < v1 ? ld_adj(d.xadj, v0 + lane) : -2;
     const unsigned up = __ballot_sync(kFull, w0 == v + 1), dn = __ballot_sync(kFull, w0 == v - 1);
     if (up | dn) {
+        if (lane == 0) linked = 1;
         const int step = lane < 16 ? 1 : -1;
         const int64_t x = lane < 16 ? (int64_t)v + lane : (int64_t)v - (lane - 15);
         const bool have = (lane < 16 ? up && lane > 0 : dn != 0) && x >= 0 && x < r.V && bit(d.R, x);
@@ -464,15 +470,18 @@ __device__ __forceinline__ void async_round(const Run<OffT> &r, const BfsDir<Off
         const int n0 = (int)min((int64_t)kLQ, s1 - bs);
         __syncthreads();
         for (int i = tid; i < n0; i += kBlock) sm.lq[0][i] = __ldcg(qv + bs + i);
-        if (tid == 0) { sm.cnt[0] = n0; sm.cnt[1] = 0; sm.flush = 0; }
+        if (tid == 0) { sm.cnt[0] = n0; sm.cnt[1] = sm.flush = sm.linked[0] = sm.linked[1] = 0; }
         __syncthreads();
-        int c = 0;
+        int c = 0, misses = 0;  // (levels in a row that looked ahead and found no link)
+        bool chain = false;
         for (int it = 0; it < kAsyncMaxLevels; ++it) {
             const int n = sm.cnt[c];
             if (n == 0) break;
+            if (chain) misses = sm.linked[(it & 1) ^ 1] ? 0 : misses + 1;
             // a frontier that widened (here, or grid-wide in the global queue)
             // goes back to the edge-balanced top-down kernel
             const bool last = it == kAsyncMaxLevels - 1 || sm.flush;
+            chain = !last && n <= kChainN && (misses < kChainMisses || it % kChainRetry == 0);
             const auto expand = [&](int64_t x0, int64_t x1) {
                 for (int64_t e = x0; e < x1; e += 4) {
                     int32_t w[4];
@@ -501,9 +510,9 @@ __device__ __forceinline__ void async_round(const Run<OffT> &r, const BfsDir<Off
                     }
                 }
             };
-            if (!last && n <= kChainN) {
+            if (chain) {
                 for (int i = tid >> 5; i < n; i += kWarps)
-                    async_chain(r, d, sm.lq[c][i], qvn, qen, qcn, pk_next, nvis, msum_next, expand);
+                    async_chain(r, d, sm.lq[c][i], qvn, qen, qcn, pk_next, nvis, msum_next, sm.linked[it & 1], expand);
             } else for (int i = tid; i < n; i += kBlock) {
                 const int32_t v = sm.lq[c][i];
                 const int64_t x0 = ld_off(d.xbeg, v), x1 = ld_off(d.xbeg, v + 1);
@@ -521,6 +530,7 @@ __device__ __forceinline__ void async_round(const Run<OffT> &r, const BfsDir<Off
             if (tid == 0) {
                 sm.cnt[c ^ 1] = min(sm.cnt[c ^ 1], kLQ);  // claims beyond the capacity went global
                 sm.cnt[c] = 0;
+                sm.linked[(it & 1) ^ 1] = 0;
                 const int64_t global_q = (int64_t)(__ldcg(pk_next) & kCountMask);
                 sm.flush = sm.cnt[c ^ 1] > kAsyncFlush || global_q > r.async_v;
             }

@@ -83,3 +83,25 @@ def test_ebbing_search(second):
                 labels, st = ctx.run_csr(csr, use_graph=graph)
                 assert np.array_equal(labels, exact)
                 assert st["giant_size"] == st["fw_size"] == 1 + leaves + second + third
+
+
+@pytest.mark.parametrize("mixed,run", [(7, 100), (8, 100), (9, 64), (31, 33), (32, 200), (33, 100), (300, 700)])
+def test_stretches_after_shuffled_ids(mixed, run):
+    """Stretches of consecutive ids with `mixed` vertices of shuffled ids between
+    them: levels that look ahead in vain, then seldom, and find links again."""
+    import oracle
+    from ispan_b200 import Context
+    from ispan_b200.graphs import from_edges
+    V = 90_000
+    rng = np.random.default_rng(mixed)
+    k = V // (mixed + run)
+    near = np.arange(k * run).reshape(k, run)
+    far = rng.permutation(np.arange(k * run, k * (run + mixed))).reshape(k, mixed)
+    ring = np.concatenate([np.concatenate([near[i], far[i]]) for i in rng.permutation(k)])
+    csr = from_edges(V, np.stack([ring, np.roll(ring, -1)], 1))
+    exact = oracle.tarjan(csr)
+    with Context(csr.V, csr.E) as ctx:
+        for graph in (False, True, True):
+            labels, st = ctx.run_csr(csr, use_graph=graph)
+            assert np.array_equal(labels, exact)
+            assert st["giant_size"] == len(ring)

@@ -160,3 +160,29 @@ def test_walks_beside_rings(line, step):
         t = time.perf_counter()
         ctx.run_csr(csr)
         assert time.perf_counter() - t < 0.1  # (the line with ids as priorities: 0.3 s and more)
+
+
+# rings of about kCycMax runs of consecutive ids (every second id, two rings
+# interleaved), and cycles of about kCycMax nodes (rings of four and single
+# vertices in turn), just below, at and above the longest walk; edges up and down
+@pytest.mark.parametrize("length", [4095, 4096, 4097, 4098])
+@pytest.mark.parametrize("down", [False, True])
+def test_longest_walks_of_runs(length, down):
+    i = np.arange(length)
+    edges = [(int(2 * a + p), int(2 * ((a + 1) % length) + p)) for p in (0, 1) for a in i] + [(0, 1)]
+    if down:
+        edges = [(b, a) for a, b in edges]
+    _check(_gadgets(6, 2 * length, edges, dag=20, seed=length, order="blocks"))
+
+
+@pytest.mark.parametrize("pairs", [2046, 2047, 2048, 2049])
+@pytest.mark.parametrize("down", [False, True])
+@pytest.mark.parametrize("order", ["up", "blocks"])
+def test_longest_walks_of_nodes(pairs, down, order):
+    edges = []
+    for k in range(pairs):
+        b, nxt = 5 * k, 5 * ((k + 1) % pairs)
+        edges += [(b, b + 1), (b + 1, b + 2), (b + 2, b + 3), (b + 3, b), (b + 3, b + 4), (b + 4, nxt)]
+    if down:
+        edges = [(b, a) for a, b in edges]
+    _check(_gadgets(5, 5 * pairs, edges, dag=20, seed=pairs, order=order))
