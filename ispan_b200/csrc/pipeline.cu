@@ -569,7 +569,7 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     // what follows the first peel, and in it the large WCCs, as conditional
     // parts of a captured graph (stage times need their events between all
     // stages, which a conditional part cannot hold)
-    const bool gates = capturing && !times && !(r.flags & ISPAN_F_EXACT_STATS);
+    const bool gates = capturing && !times;
     cudaGraphNode_t if_left = nullptr, if_large = nullptr;
     if (gates && (e = if_gate(s, &x.gate_left))) return e;
     const bool pair = pair_searches(c, r);
@@ -685,8 +685,10 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     cy.single = c->members;
     cy.q[0] = c->members;
     cy.q[1] = c->roots;
-    if ((e = launch_coop(k_cycles<OffT>, c->g_coop[5], s, r, x, cy))) return e;
-    prev_plain = false;
+    if (r.V >= kCycMin) {  // (smaller graphs never have as many residual vertices)
+        if ((e = launch_coop(k_cycles<OffT>, c->g_coop[5], s, r, x, cy))) return e;
+        prev_plain = false;
+    }
     PK((k_wcc_init<OffT>), G, kBlock, r, x, 0, (const int32_t *)cy.rep);
     PK((k_wcc_hook<OffT>), G, kBlock, r, x, 0, 0);
     PK((k_wcc_compress<OffT>), G, kBlock, r, x, 0);
@@ -708,8 +710,10 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
         if ((e = if_begin(s, c->stream_if[1], x.gate_large, &if_large))) return e;
         s = c->stream_if[1];
     }
-    if ((e = launch_coop(k_super<OffT>, c->g_coop[6], s, r, x, cy))) return e;
-    prev_plain = false;
+    if (r.V >= kCycMin) {
+        if ((e = launch_coop(k_super<OffT>, c->g_coop[6], s, r, x, cy))) return e;
+        prev_plain = false;
+    }
     if (c->tuning.color_compact >= 0 && r.V >= 4 * kCmpMin) {  // (smaller graphs never qualify)
         // the large WCCs' subgraph in dense ids (compact.cuh), then the
         // colouring on it; the input-graph form returns at once if it was built
