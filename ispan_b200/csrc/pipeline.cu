@@ -685,7 +685,11 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
     cy.single = c->members;
     cy.q[0] = c->members;
     cy.q[1] = c->roots;
-    if (r.V >= kCycMin) {  // (smaller graphs never have as many residual vertices)
+    // smaller graphs never have as many residual vertices: not launched directly
+    // (in a captured graph's conditional part the nodes cost nothing; R-MAT scale
+    // 10 takes 71-73 us a call with them and 74-76 without)
+    const bool cycles = gates || r.V >= kCycMin;
+    if (cycles) {
         if ((e = launch_coop(k_cycles<OffT>, c->g_coop[5], s, r, x, cy))) return e;
         prev_plain = false;
     }
@@ -710,7 +714,7 @@ static cudaError_t enqueue(ispan_ctx *c, Run<OffT> r, Ext<OffT> x, bool times, b
         if ((e = if_begin(s, c->stream_if[1], x.gate_large, &if_large))) return e;
         s = c->stream_if[1];
     }
-    if (r.V >= kCycMin) {
+    if (cycles) {
         if ((e = launch_coop(k_super<OffT>, c->g_coop[6], s, r, x, cy))) return e;
         prev_plain = false;
     }
